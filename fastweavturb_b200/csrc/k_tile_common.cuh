@@ -195,7 +195,8 @@ __device__ __forceinline__ void tile_epilogue(long long (*acc)[kAccN], int N, in
 {
     const int tid = threadIdx.x;
     const double inv = 1.0 / scale;
-    const bool full = (x0 + TX <= N) && (y0 + TY <= N) && (z0 + TZ <= zlim);
+    // 16-byte stores need rows that start on 16 bytes: N a multiple of 4
+    const bool full = (x0 + TX <= N) && (y0 + TY <= N) && (z0 + TZ <= zlim) && (N & 3) == 0;
     if (full) {
         for (int q4 = tid; q4 < TP / 4; q4 += blockDim.x) {
             const int p = 4 * q4;
