@@ -5,6 +5,57 @@
 
 namespace fwt {
 
+// e^x = 2^(x log2 e) and 1/sqrt(x) by one hardware operation each, subnormal numbers flushed:
+// the profile's exponent lies in [-Rtube_ratio^2 / 2, 0] and |c'|^2 is of order one, so neither
+// an operand nor a result is subnormal, and the scaling that guards subnormals (three
+// instructions each in the innermost loop) is left out.
+__device__ __forceinline__ float exp_hw(float x)
+{
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.4426950408889634f));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_hw(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Two FP32 numbers in one 64-bit register, for sm_100a's packed FP32 arithmetic: one issue slot
+// does two multiply-adds, each rounded as the scalar instruction rounds it.
+struct f32x2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ f32x2 pk(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpk(f32x2 p, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
 // ---------------------------------------------------------------------------- FP64 reference
 // The reference's inner body (tube.f90:806-892) split in two: the acceptance tests
 // (tube.f90:806-818) and the vorticity of an accepted point (tube.f90:819-892), statement for
@@ -452,6 +503,16 @@ __device__ __forceinline__ int point_f32(const SegF &G, int ii, int jj, int kk, 
 
 constexpr int kNoWrap = 1 << 20;   // SegRec::kq[0] marker: the record never needs the wrap logic
 
+// Whether the first wrap of x - c(zeta) is by at most one period for every |P| <= pb: kq in
+// {-1, 0, 1} and, for kq = +-1, no wrap of the spline position in the same direction.
+__device__ __forceinline__ bool wraps_cancel(int kq, float pb, float thi, float tlo)
+{
+    if (kq > 1 || kq < -1) return false;
+    if (kq == 1) return thi > pb * 1.01f + 1e-5f;
+    if (kq == -1) return tlo < -pb * 1.01f - 1e-5f;
+    return true;
+}
+
 // Compact FP32 record of one sub-segment for the tile kernel (224 bytes, 16-byte aligned):
 // the local frame of SegF taken at the box origin box_lo, the line constants, and the box.
 struct __align__(16) SegRec {
@@ -502,27 +563,31 @@ __device__ __forceinline__ void segrec_from(const SegF &G, const SubSeg &S, SegR
     // per-record constants of the constant-core profile (tube.f90:845-847 with sigma = smin)
     const float s2 = G.smin * G.smin;
     R.inv2s2 = 0.5f / s2;
-    R.ftd = __expf(-G.R2 * R.inv2s2);   // the same exponential as the per-point term
+    R.ftd = exp_hw(-G.R2 * R.inv2s2);   // the same exponential as the per-point term
     R.amp = G.Gamma * (0.159154943091895336f / s2);
-    // No-wrap flag (kq[0] = kNoWrap): for every point that passes the tests, |W| <= Wm, so
-    // |P| stays clear of both wrap thresholds and |x - c| < pi; the wrap bookkeeping of
-    // point_rec then reduces to x - c = d0 - P.  An accepted point has 0 <= t0 <= dl + Rt
-    // (bends below 45 degrees, checked below) and a distance below Rt from the chord line, so
-    // |d0| <= sqrt((dl + Rt)^2 + Rt^2) and |x - c| <= |d0| + |P|.
+    // No-wrap flag (kq[0] = kNoWrap): the two wraps of vort_w leave x - c = d0 - P as it is for
+    // every point that passes the tests.  An accepted point lies between the planes: 0 <= t0 <=
+    // dl + Rt tan(bend) (bends below 41 degrees, checked below), and within Rt of the chord line,
+    // so |d0| <= sqrt(t0max^2 + Rt^2) and |x - c| <= |d0| + |P|, |P| <= pb per axis.  The first
+    // wrap moves x - c by n1 = kq + (P >= thi) - (P < tlo) periods and the second takes one
+    // period back when |n1| = 1 and |x - c| < pi; n1 beyond +-1 needs a second wrap of the
+    // spline in the direction of kq, which the bound on P rules out.
     const float dl = sqrtf(G.dci[0] * G.dci[0] + G.dci[1] * G.dci[1] + G.dci[2] * G.dci[2]);
-    const float Wm = (dl + G.Rt) * fabsf(G.g) * 1.01f;
-    bool nowrap = true;
+    const float cth = G.tc0[0] * G.tc1[0] + G.tc0[1] * G.tc1[1] + G.tc0[2] * G.tc1[2];
+    const float s0 = G.tc0[1] * G.tc1[2] - G.tc0[2] * G.tc1[1], s1 = G.tc0[2] * G.tc1[0] - G.tc0[0] * G.tc1[2],
+                s2_ = G.tc0[0] * G.tc1[1] - G.tc0[1] * G.tc1[0];
+    bool nowrap = cth >= 0.75f;
+    const float t0max = (dl + G.Rt * sqrtf(s0 * s0 + s1 * s1 + s2_ * s2_) / fmaxf(cth, 0.75f)) * 1.01f;
+    const float Wm = t0max * fabsf(G.g);
     float pmax = 0.0f;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const float *b = G.b[d];
         const float pb = Wm * (fabsf(b[0]) + Wm * (fabsf(b[1]) + Wm * (fabsf(b[2]) + Wm * (fabsf(b[3]) + Wm * fabsf(b[4])))));
         pmax = fmaxf(pmax, pb);
-        if (G.kq[d] != 0 || !(G.thi[d] > pb * 1.01f + 1e-5f) || !(G.tlo[d] < -pb * 1.01f - 1e-5f)) nowrap = false;
+        if (!wraps_cancel(G.kq[d], pb, G.thi[d], G.tlo[d])) nowrap = false;
     }
-    if (sqrtf((dl + G.Rt) * (dl + G.Rt) + G.R2) + pmax > 3.0f) nowrap = false;
-    // t0 <= dl + Rt tan(bend) <= dl + Rt holds for bends below 45 degrees
-    if (G.tc0[0] * G.tc1[0] + G.tc0[1] * G.tc1[1] + G.tc0[2] * G.tc1[2] < 0.75f) nowrap = false;
+    if (!(sqrtf(t0max * t0max + G.R2) + 1.7321f * pmax < 3.0f)) nowrap = false;
     if (nowrap) R.kq[0] = kNoWrap;
 }
 
@@ -558,7 +623,9 @@ __device__ __forceinline__ int rec_classify(const RecT &R, float d0x, float d0y,
 // w sum_k b_k D_k, D_k = ((zb + w)^k - zb^k) / w, which keeps its relative accuracy however
 // large zb is.  The wrap decisions still use P(W), which needs no such accuracy: a decision
 // moved by rounding is undone by the final single wrap.
-template <bool General, bool Delta, typename RecT>
+//
+// Wrap = false: the caller knows that the record carries the no-wrap flag.
+template <bool General, bool Delta, bool Wrap = true, typename RecT>
 __device__ __forceinline__ void vort_w(const RecT &R, float d0x, float d0y, float d0z, float zb, float w, float R2,
                                        float out[3], float &cond)
 {
@@ -594,7 +661,7 @@ __device__ __forceinline__ void vort_w(const RecT &R, float d0x, float d0y, floa
     float xc[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) xc[d] = d0[d] - Q[d];
-    if (R.kq[0] != kNoWrap) {
+    if (Wrap && R.kq[0] != kNoWrap) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             int n = R.kq[d] + (P[d] >= R.thi[d] ? 1 : 0) - (P[d] < R.tlo[d] ? 1 : 0);
@@ -605,10 +672,10 @@ __device__ __forceinline__ void vort_w(const RecT &R, float d0x, float d0y, floa
         }
     }
     const float rho2 = xc[0] * xc[0] + xc[1] * xc[1] + xc[2] * xc[2];
-    const float in1 = rsqrtf(c1[0] * c1[0] + c1[1] * c1[1] + c1[2] * c1[2]);
+    const float in1 = rsqrt_hw(c1[0] * c1[0] + c1[1] * c1[1] + c1[2] * c1[2]);
     const float T[3] = {c1[0] * in1, c1[1] * in1, c1[2] * in1};
     if constexpr (!General) {
-        const float tp = (__expf(-rho2 * R.inv2s2) - R.ftd) * R.amp;
+        const float tp = (exp_hw(-rho2 * R.inv2s2) - R.ftd) * R.amp;
         out[0] = tp * T[0];
         out[1] = tp * T[1];
         out[2] = tp * T[2];
@@ -625,7 +692,7 @@ __device__ __forceinline__ void vort_w(const RecT &R, float d0x, float d0y, floa
         const float sigma = fmaf(R.A, sn + 1.0f, R.smin);
         const float s2 = sigma * sigma;
         const float inv2s2 = 0.5f / s2;
-        const float tp = (__expf(-rho2 * inv2s2) - __expf(-R2 * inv2s2)) * (0.159154943f / s2) * R.Gamma;
+        const float tp = (exp_hw(-rho2 * inv2s2) - exp_hw(-R2 * inv2s2)) * (0.159154943f / s2) * R.Gamma;
         const float dsds = R.q * cs * in1 * R.Linv;
         const float rho = sqrtf(rho2);
         const float X[3] = {c1[1] * c2[2] - c1[2] * c2[1], c1[2] * c2[0] - c1[0] * c2[2], c1[0] * c2[1] - c1[1] * c2[0]};
@@ -657,11 +724,11 @@ __device__ __forceinline__ void vort_w(const RecT &R, float d0x, float d0y, floa
 
 // The vorticity of tube.f90:819-892 for a point that passed rec_classify with argument t0
 // (sub-segment record: W = t0 g), and its curved-branch amplification.
-template <bool General, typename RecT>
+template <bool General, bool Wrap = true, typename RecT>
 __device__ __forceinline__ void rec_vorticity(const RecT &R, float d0x, float d0y, float d0z, float t0, float out[3],
                                               float &cond)
 {
-    vort_w<General, false>(R, d0x, d0y, d0z, 0.0f, t0 * R.g, R.R2, out, cond);
+    vort_w<General, false, Wrap>(R, d0x, d0y, d0z, 0.0f, t0 * R.g, R.R2, out, cond);
 }
 
 int launch_walk(Ctx *c, const CenterlineBatch &B, unsigned long long *d_acc);

@@ -189,18 +189,26 @@ __global__ void __launch_bounds__(kBuildThreads, 6) piece_build_kernel(
     PieceRec &R = rec[pc];
     int blo[3] = {1 << 30, 1 << 30, 1 << 30}, bhi[3] = {-(1 << 30), -(1 << 30), -(1 << 30)};
     int b0[3] = {0, 0, 0};   // chord 0's box origin: the reference of s_box
-    double Rmax = 0.0, dlen = 0.0;
-    float bendmin = 1.0f, Wm = 0.0f, cmax = 0.0f;
+    float bendmin = 1.0f, Wm = 0.0f, cmax = 0.0f, dmx = 0.0f, lprev = 0.0f, Rprev = 0.0f, gprev = 0.0f;
     double tprev[3] = {0.0, 0.0, 0.0};
     walk([&](int jj, const double *ch, double nd, const double *pj, const int *lo3, const int *hi3, double s0,
              double s1, double Rt) {
         const double inv = 1.0 / nd;
         const double tc[3] = {ch[0] * inv, ch[1] * inv, ch[2] * inv};
-        if (jj > 0) bendmin = fminf(bendmin, (float)(tc[0] * tprev[0] + tc[1] * tprev[1] + tc[2] * tprev[2]));
+        if (jj > 0) {
+            // the previous chord's accepted points lie between its planes, within its Rtube:
+            // 0 <= t <= |chord| + Rtube tan(bend)
+            const float cth = (float)(tc[0] * tprev[0] + tc[1] * tprev[1] + tc[2] * tprev[2]);
+            const float sx = (float)(tprev[1] * tc[2] - tprev[2] * tc[1]), sy = (float)(tprev[2] * tc[0] - tprev[0] * tc[2]),
+                        sz = (float)(tprev[0] * tc[1] - tprev[1] * tc[0]);
+            bendmin = fminf(bendmin, cth);
+            const float tm = (lprev + Rprev * sqrtf(sx * sx + sy * sy + sz * sz) / fmaxf(cth, 0.75f)) * 1.01f;
+            Wm = fmaxf(Wm, s_zoff[tid][jj - 1] * 1.01f + tm * gprev);
+            dmx = fmaxf(dmx, sqrtf(tm * tm + Rprev * Rprev));
+        }
         tprev[0] = tc[0];
         tprev[1] = tc[1];
         tprev[2] = tc[2];
-        dlen = fmax(dlen, sqrt(pj[0] * pj[0] + pj[1] * pj[1] + pj[2] * pj[2]));
         const float ck = (float)(tc[0] * pj[0] + tc[1] * pj[1] + tc[2] * pj[2]);
         R.pl[jj] = make_float4((float)tc[0], (float)tc[1], (float)tc[2], ck);
         cmax = fmaxf(cmax, fabsf(ck));
@@ -209,7 +217,6 @@ __global__ void __launch_bounds__(kBuildThreads, 6) piece_build_kernel(
 #pragma unroll
         for (int k = 0; k < 3; ++k) s_pj[tid][jj][k] = pj[k];
         if (jj == n) return;
-        Rmax = fmax(Rmax, Rt);
         if (jj == 0) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) b0[k] = lo3[k];
@@ -224,7 +231,9 @@ __global__ void __launch_bounds__(kBuildThreads, 6) piece_build_kernel(
         }
         const float g = (float)((s1 - s0) * L * inv);
         R.chq[jj] = make_float4(g, (float)(Rt * Rt), 0.0f, 0.0f);
-        Wm = fmaxf(Wm, (zoff + (float)(nd + Rt) * fabsf(g)) * 1.01f);
+        lprev = (float)nd;
+        Rprev = (float)Rt;
+        gprev = fabsf(g);
     });
     double X0[3];
 #pragma unroll
@@ -284,10 +293,10 @@ __global__ void __launch_bounds__(kBuildThreads, 6) piece_build_kernel(
         const float pb =
             Wm * (fabsf(bb[0]) + Wm * (fabsf(bb[1]) + Wm * (fabsf(bb[2]) + Wm * (fabsf(bb[3]) + Wm * fabsf(bb[4])))));
         pmax = fmaxf(pmax, pb);
-        if (R.kq[k] != 0 || !(R.thi[k] > pb * 1.01f + 1e-5f) || !(R.tlo[k] < -pb * 1.01f - 1e-5f)) nowrap = false;
+        if (!wraps_cancel(R.kq[k], pb, R.thi[k], R.tlo[k])) nowrap = false;
     }
-    // as segrec_from: every accepted point keeps |P| clear of the wrap thresholds and |x - c| < pi
-    if (((float)dlen + 2.0f * (float)Rmax) * 1.7321f + pmax > 3.0f) nowrap = false;
+    // as segrec_from: |x - c| <= |x - sample j| + |P(zb + w) - P(zb)| < pi for every accepted point
+    if (!(dmx + 2.0f * 1.7321f * pmax < 3.0f)) nowrap = false;
     if (bendmin < 0.75f) nowrap = false;
     if (nowrap) R.kq[0] = kNoWrap;
     // core size sigma(zeta) = smin + A (sin(omega zeta) + 1), zeta = s_j0 + W / Len
@@ -310,7 +319,7 @@ __global__ void __launch_bounds__(kBuildThreads, 6) piece_build_kernel(
     const double rt = Rtube_ratio * P.sigma_min;
     const float s2 = R.smin * R.smin;
     R.inv2s2 = 0.5f / s2;
-    R.ftd = __expf(-(float)(rt * rt) * R.inv2s2);   // the same exponential as the per-point term
+    R.ftd = exp_hw(-(float)(rt * rt) * R.inv2s2);   // the same exponential as the per-point term
     R.amp = R.Gamma * (0.159154943091895336f / s2);
     R.pad1 = 0;
 }

@@ -21,6 +21,7 @@
 #include <cstdio>
 #include <cstdlib>
 
+#include "k_block.cuh"
 #include "k_deposit.cuh"
 #include "k_tile_common.cuh"
 
@@ -461,6 +462,161 @@ __global__ void __launch_bounds__(kDepThreads, F64 ? 2 : 3) deposit_tile_kernel(
         tile_epilogue(acc, N, x0, y0, z0, zs, zlim, scale, (float *)wx, (float *)wy, (float *)wz);
 }
 
+// Sub-segment records through deposit_block_kernel: a block is culled by the record's two planes
+// and its cylinder (the bounds of tile_may_hit), a point takes rec_classify's tests.
+struct SegBlocks {
+    using Rec = SegRec;
+    static constexpr int kChunk = 64;   // 14 KB of records per buffer
+    static constexpr int kCtas = 3;
+    // The culls' data record by record, and the constants of the packed evaluation, each twice (a
+    // packed operand is a register pair, so a scalar would be copied for every use): b[15], g,
+    // -inv2s2, -ftd, amp and a pad.  The plane tests share x and y between the packed points and
+    // stay scalar; doubling their constants too made the kernel shared-memory bound.
+    struct Prep {
+        f32x2 c[kChunk][20];
+        float4 org[kChunk];                  // tile origin from box_lo (grid points); plane_eps
+        float b[3][kChunk];                  // tile origin minus ci0
+        float tc0[3][kChunk], tc1[3][kChunk];
+        float k1[kChunk], Rt[kChunk];        // tc1 . dci; Rtube
+        float dl[3][kChunk], ext[3][kChunk]; // tile origin from box_lo, box extent (grid points)
+        bool wrap[kChunk];                   // the record needs the periodic bookkeeping
+    };
+    // four threads per record
+    static __device__ __forceinline__ void prepare(Prep &P, int t, int part, const SegRec &R, uint32_t img, int N, int x0,
+                                                   int y0, int z0)
+    {
+        if (part == 0) {
+            const int tl[3] = {x0, y0, z0};
+            const int m[3] = {(int)(img % 3) - 1, (int)((img / 3) % 3) - 1, (int)(img / 9) - 1};
+            int ext[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const float dl = (float)(tl[d] + m[d] * N - (R.box_lo[d] - 1));
+                ext[d] = R.box_hi[d] - R.box_lo[d];
+                P.b[d][t] = fmaf(dl, R.dx, R.off[d]);
+                P.dl[d][t] = dl;
+                P.ext[d][t] = (float)ext[d];
+            }
+            P.org[t] = make_float4(P.dl[0][t], P.dl[1][t], P.dl[2][t], plane_eps(R.off, ext, R.dx, R.dci));
+        } else if (part == 1) {
+            float k1 = 0.0f;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                P.tc0[d][t] = R.tc0[d];
+                P.tc1[d][t] = R.tc1[d];
+                k1 = fmaf(R.tc1[d], R.dci[d], k1);
+            }
+            P.k1[t] = k1;
+            P.Rt[t] = sqrtf(R.R2);
+            P.wrap[t] = R.kq[0] != kNoWrap;
+            P.c[t][16] = pk(-R.inv2s2, -R.inv2s2);
+            P.c[t][17] = pk(-R.ftd, -R.ftd);
+            P.c[t][18] = pk(R.amp, R.amp);
+        } else {
+            const int h = part - 2;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float v = h == 0 ? R.b[i] : (i < 7 ? R.b[8 + (i < 7 ? i : 0)] : R.g);
+                P.c[t][8 * h + i] = pk(v, v);
+            }
+        }
+    }
+    static __device__ __forceinline__ int may_hit(const Prep &P, int k, float dx, float bx, float by, float bz)
+    {
+        const float Rt = P.Rt[k];
+        const float hx = 0.5f * (kBX - 1) * dx, hy = 0.5f * (kBY - 1) * dx, hz = 0.5f * (kBZ - 1) * dx;
+        const float hn = kBlockHalfDiag * dx;
+        const float cx = fmaf(bx, dx, P.b[0][k]) + hx, cy = fmaf(by, dx, P.b[1][k]) + hy,
+                    cz = fmaf(bz, dx, P.b[2][k]) + hz;
+        const float e = 1e-3f * (hn + Rt + dx);   // slack for the rounding of the bounds
+        const float ax = P.tc0[0][k], ay = P.tc0[1][k], az = P.tc0[2][k];
+        const float t0c = fmaf(cz, az, fmaf(cy, ay, cx * ax));
+        const float t0h = fmaf(hz, fabsf(az), fmaf(hy, fabsf(ay), hx * fabsf(ax)));
+        const float ex = P.tc1[0][k], ey = P.tc1[1][k], ez = P.tc1[2][k];
+        const float t1c = fmaf(cz, ez, fmaf(cy, ey, cx * ex)) - P.k1[k];
+        const float t1h = fmaf(hz, fabsf(ez), fmaf(hy, fabsf(ey), hx * fabsf(ex)));
+        const float d2 = fmaf(-t0c, t0c, fmaf(cz, cz, fmaf(cy, cy, cx * cx)));
+        const float rr = Rt + hn + e;
+        if (!(t0c + t0h >= -e && t1c - t1h <= e && d2 <= rr * rr)) return kMiss;
+        if (P.wrap[k]) return kWrapped;
+        const float ux = bx + P.dl[0][k], uy = by + P.dl[1][k], uz = bz + P.dl[2][k];
+        return ux >= 0.0f && uy >= 0.0f && uz >= 0.0f && ux + (kBX - 1) <= P.ext[0][k] && uy + (kBY - 1) <= P.ext[1][k] &&
+                       uz + (kBZ - 1) <= P.ext[2][k]
+                   ? kPlain
+                   : kBoxed;
+    }
+    // The lane's two points, (lx, ly, lz) and (lx, ly, lz + 1) in the tile.
+    template <bool General, int Form, typename Sink>
+    static __device__ __forceinline__ void visit(const Prep &P, const SegRec &R, int k, float dx, float lx, float ly,
+                                                 float lz, bool in0, bool in1, Sink &&sink)
+    {
+        const float4 *q = reinterpret_cast<const float4 *>(&R);
+        const float4 o = q[0], n0 = q[1], n1 = q[2], dc = q[3], fr = P.org[k];
+        const float fx = lx + fr.x, fy = ly + fr.y, f0 = lz + fr.z, f1 = f0 + 1.0f, pe = fr.w;
+        const float x = fmaf(fx, dx, o.x), y = fmaf(fy, dx, o.y), za = fmaf(f0, dx, o.z), zb = fmaf(f1, dx, o.z);
+        // rec_classify, without its early exits: a point within pe of a plane is left to the FP64
+        // tests whichever side it lies on, so the two planes are judged by the smaller margin
+        const float txy = fmaf(y, n0.y, x * n0.x);
+        const float ta = fmaf(za, n0.z, txy), tb = fmaf(zb, n0.z, txy);
+        const float exy = fmaf(y - dc.y, n1.y, (x - dc.x) * n1.x);
+        const float ua = fmaf(za - dc.z, n1.z, exy), ub = fmaf(zb - dc.z, n1.z, exy);
+        const float rxy = fmaf(y, y, x * x);
+        const float ra = fmaf(-ta, ta, fmaf(za, za, rxy)), rb = fmaf(-tb, tb, fmaf(zb, zb, rxy));
+        const float ma = fminf(ta, -ua), mb = fminf(tb, -ub);
+        bool ok0 = ma >= -pe && ra < n0.w, ok1 = mb >= -pe && rb < n0.w;
+        if constexpr (Form != kPlain) {
+            ok0 = ok0 && in0;
+            ok1 = ok1 && in1;
+        }
+        if (!__any_sync(0xffffffffu, ok0 || ok1)) return;
+        if constexpr (Form != kPlain) {   // the reference visits the points of the record's box only
+            const float ez = P.ext[2][k];
+            const bool xy = fx >= 0.0f && fy >= 0.0f && fx <= P.ext[0][k] && fy <= P.ext[1][k];
+            ok0 = ok0 && xy && f0 >= 0.0f && f0 <= ez;
+            ok1 = ok1 && xy && f1 >= 0.0f && f1 <= ez;
+        }
+        const bool sure0 = ma >= pe, sure1 = mb >= pe;
+        f32x2 v[3];
+        float cond0 = 1.0f, cond1 = 1.0f;
+        if constexpr (General || Form == kWrapped) {
+            float a[3], b[3];
+            rec_vorticity<General, Form == kWrapped>(R, x, y, za, ta, a, cond0);
+            rec_vorticity<General, Form == kWrapped>(R, x, y, zb, tb, b, cond1);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) v[d] = pk(a[d], b[d]);
+        } else {
+            // vort_w<false, false, false> (constant core, no twist, no wrap), operation for operation
+            const f32x2 *c = P.c[k];
+            const f32x2 W = mul2(pk(ta, tb), c[15]);
+            float wa, wb;
+            unpk(W, wa, wb);
+            f32x2 xc[3], c1[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const f32x2 *b = c + 5 * d;
+                const f32x2 h3 = fma2(W, b[4], b[3]);
+                const f32x2 h2 = fma2(W, h3, b[2]);
+                const f32x2 h1 = fma2(W, h2, b[1]);
+                const f32x2 h0 = fma2(W, h1, b[0]);
+                c1[d] = fma2(W, fma2(W, fma2(W, fma2(W, b[4], h3), h2), h1), h0);
+                float ha, hb;
+                unpk(h0, ha, hb);
+                xc[d] = pk(fmaf(-wa, ha, d == 0 ? x : (d == 1 ? y : za)), fmaf(-wb, hb, d == 0 ? x : (d == 1 ? y : zb)));
+            }
+            const f32x2 rho2 = fma2(xc[2], xc[2], fma2(xc[1], xc[1], mul2(xc[0], xc[0])));
+            const f32x2 n2 = fma2(c1[2], c1[2], fma2(c1[1], c1[1], mul2(c1[0], c1[0])));
+            float na, nb, ea, eb;
+            unpk(n2, na, nb);
+            const f32x2 in1_ = pk(rsqrt_hw(na), rsqrt_hw(nb));
+            unpk(mul2(rho2, c[16]), ea, eb);
+            const f32x2 tp = mul2(add2(pk(exp_hw(ea), exp_hw(eb)), c[17]), c[18]);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) v[d] = mul2(tp, mul2(c1[d], in1_));
+        }
+        sink(ok0 && sure0, ok1 && sure1, ok0 && !sure0, ok1 && !sure1, 0, 0, v, cond0, cond1);
+    }
+};
+
 
 RedoCtx redo_ctx(const Ctx *c, const CenterlineBatch &B, double scale, bool pieces)
 {
@@ -651,6 +807,7 @@ int launch_tile(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
     const int ntz = c->slab_nz ? c->slab_nz / TZ : (N + TZ - 1) / TZ;
     const int64_t ntiles = (int64_t)ntx * nty * ntz;
     if (B.nsub >= ((int64_t)1 << 26)) return fail(FWT_E_RANGE, "sub-segment batch exceeds 2^26");
+    const bool f64 = c->p.precision == 64;
     if (!B.rec) return fail(FWT_E_STATE, "tile deposition needs the FP32 sub-segment records");
     Ctx &C = *c;
     // scratch[20]: pair counts/offsets (nsub+1 int64), [21]: key,val (2 x npairs u32),
@@ -701,7 +858,6 @@ int launch_tile(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
     }
 
     const size_t n3 = field_elems(c);
-    const bool f64 = c->p.precision == 64;
     const size_t rb = f64 ? 8 : 4;
     char *w = (char *)c->b_w.p;
     void *wx = w, *wy = w + n3 * rb, *wz = w + 2 * n3 * rb;
@@ -713,6 +869,10 @@ int launch_tile(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
     rctx.tally = (unsigned long long *)((char *)C.scratch[19].p + 64);
     DeferList D{};
     if (!f64) FWT_TRY(defer_list(c, npairs, c->defer_per_pair, D));
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
+    const unsigned parts = (unsigned)block_parts(ntiles, sms, SegBlocks::kCtas);
+    const double dxg = kPi2 / N;   // as the records' dx
     auto launch = [&](const DeferList &L) -> int {
 #define FWT_TILE_LAUNCH(G, A, F)                                                                          \
     do {                                                                                                  \
@@ -724,14 +884,24 @@ int launch_tile(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
     } while (0)
         const unsigned grid = (unsigned)(std::min<int64_t>(ntiles, L.w1) - L.w0);
         const int m = kt_begin(c, KT_DEPOSIT);
+#define FWT_BLOCK_LAUNCH(G, A)                                                                             \
+    do {                                                                                                   \
+        FWT_CUDA(cudaFuncSetAttribute(deposit_block_kernel<SegBlocks, G, A>,                               \
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem<SegBlocks>())); \
+        deposit_block_kernel<SegBlocks, G, A><<<grid * parts, kDepThreads, block_smem<SegBlocks>(), c->stream>>>( \
+            B.rec, N, ntx, nty, tz0, (int)parts, d_toff, d_list, scale, (float *)wx, (float *)wy, (float *)wz, d_err, \
+            rctx.zs, rctx.zs + rctx.nz, (float)dxg, rctx.tally, L);                                       \
+        FWT_CUDA(cudaGetLastError());                                                                      \
+    } while (0)
         if (f64) {
             // the FP64 path evaluates every pair in FP64: the General distinction is only the FP32 one
             if (accumulate) FWT_TILE_LAUNCH(true, true, true); else FWT_TILE_LAUNCH(true, false, true);
         } else if (general) {
-            if (accumulate) FWT_TILE_LAUNCH(true, true, false); else FWT_TILE_LAUNCH(true, false, false);
+            if (accumulate) FWT_BLOCK_LAUNCH(true, true); else FWT_BLOCK_LAUNCH(true, false);
         } else {
-            if (accumulate) FWT_TILE_LAUNCH(false, true, false); else FWT_TILE_LAUNCH(false, false, false);
+            if (accumulate) FWT_BLOCK_LAUNCH(false, true); else FWT_BLOCK_LAUNCH(false, false);
         }
+#undef FWT_BLOCK_LAUNCH
 #undef FWT_TILE_LAUNCH
         kt_end(c, m);
         c->launches += 1;
