@@ -60,8 +60,12 @@ constexpr size_t block_smem()
     return kAccBytes + sizeof(BlockStage<Policy>);
 }
 
+// Constant-core lines without a twist (sigma_ratio = 1, eta = 0): the vorticity has no
+// curvature term, so no pair is deferred for its conditioning.  (Lines with a varying core take
+// deposit_tile_kernel: their vorticity is five times the work, and is better evaluated with all
+// lanes busy from a queue than by the third of a block's lanes that hold accepted points.)
 // One CTA per tile part: D.w0 + blockIdx.x / parts is the tile; parts (1 or 2) cut it along z.
-template <class Policy, bool General, bool Accumulate>
+template <class Policy, bool Accumulate>
 __global__ void __launch_bounds__(kDepThreads, Policy::kCtas) deposit_block_kernel(
     const typename Policy::Rec *__restrict__ rec, int N, int ntx, int nty, int tz0, int parts,
     const int64_t *__restrict__ tile_off, const uint32_t *__restrict__ list, double scale, float *__restrict__ wx,
@@ -136,8 +140,7 @@ __global__ void __launch_bounds__(kDepThreads, Policy::kCtas) deposit_block_kern
     // an emit-only pass lists the deferred pairs again and discards its sums
     const float fscale = D.emit_only ? 0.0f : (float)scale;
     unsigned nacc = 0;       // pairs evaluated by this lane
-    bool over = false;       // General: a contribution beyond the fixed-point range
-    f32x2 poison = pk(0.0f, 0.0f);   // constant core: turns NaN with any contribution that is not finite
+    f32x2 poison = pk(0.0f, 0.0f);   // turns NaN with any contribution that is not finite
     const int plx = lane & 3, ply = (lane >> 2) & 3, plz = 2 * (lane >> 4);
     const f32x2 zero2 = pk(0.0f, 0.0f);
     uint32_t phases = 0u;    // bit b: parity of buffer b's next wait
@@ -170,49 +173,32 @@ __global__ void __launch_bounds__(kDepThreads, Policy::kCtas) deposit_block_kern
             // one record against the block's points: test, evaluate, add (every lane computes;
             // points that are not accepted add zero)
             auto one = [&](int k, auto form) {
-                Policy::template visit<General, decltype(form)::value>(
+                Policy::template visit<decltype(form)::value>(
                     S.prep, S.rec[b][k], k, dx, flx, fly, flz, in0, in1,
-                    [&](bool ok0, bool ok1, bool dec0, bool dec1, int chord0, int chord1, const f32x2 *v, float cond0,
-                        float cond1) {
+                    [&](bool ok0, bool ok1, bool dec0, bool dec1, const f32x2 *v) {
                         // dec: left to the reference's FP64 tests
-                        bool f0 = dec0, f1 = dec1;
                         nacc += ok0;
                         nacc += ok1;
-                        if (General) {
-                            const bool bad0 = ok0 && !(cond0 <= kRedoCond), bad1 = ok1 && !(cond1 <= kRedoCond);
-                            f0 = f0 || bad0;
-                            f1 = f1 || bad1;
-                            ok0 = ok0 && !bad0;
-                            ok1 = ok1 && !bad1;
-                        }
                         const f32x2 fs = pk(ok0 ? fscale : 0.0f, ok1 ? fscale : 0.0f);
                         const f32x2 s0 = mul2(v[0], fs), s1 = mul2(v[1], fs), s2 = mul2(v[2], fs);
                         float s00, s01, s02, s10, s11, s12;
                         unpk(s0, s00, s10);
                         unpk(s1, s01, s11);
                         unpk(s2, s02, s12);
-                        if (General) {
-                            const float fmaxq = 4.0e18f;
-                            over = over || !(fabsf(s00) < fmaxq && fabsf(s01) < fmaxq && fabsf(s02) < fmaxq &&
-                                             fabsf(s10) < fmaxq && fabsf(s11) < fmaxq && fabsf(s12) < fmaxq);
-                        } else {
-                            // |tp T| <= amp, and amp times the scale is at most 2^44 by the choice of
-                            // the scale: only a value that is not a number can leave the range, and
-                            // then all three components are none (they share tp / |c'|)
-                            poison = fma2(s0, zero2, poison);
-                        }
+                        // |tp T| <= amp, and amp times the scale is at most 2^44 by the choice of the
+                        // scale: only a value that is not a number can leave the fixed-point range, and
+                        // then all three components are none (they share tp / |c'|)
+                        poison = fma2(s0, zero2, poison);
                         a00 += __float2ll_rn(s00);
                         a01 += __float2ll_rn(s01);
                         a02 += __float2ll_rn(s02);
                         a10 += __float2ll_rn(s10);
                         a11 += __float2ll_rn(s11);
                         a12 += __float2ll_rn(s12);
-                        if (__any_sync(0xffffffffu, f0 || f1)) {
-                            const uint32_t id = S.id[b][k] & ((1u << 26) - 1u);
-                            defer_push(D, lane, f0, id | ((uint32_t)chord0 << 26) | (dec0 ? kDeferDecide : 0u), x0 + lx,
-                                       y0 + ly, z0 + lz);
-                            defer_push(D, lane, f1, id | ((uint32_t)chord1 << 26) | (dec1 ? kDeferDecide : 0u), x0 + lx,
-                                       y0 + ly, z0 + lz + 1);
+                        if (__any_sync(0xffffffffu, dec0 || dec1)) {
+                            const uint32_t id = (S.id[b][k] & ((1u << 26) - 1u)) | kDeferDecide;
+                            defer_push(D, lane, dec0, id, x0 + lx, y0 + ly, z0 + lz);
+                            defer_push(D, lane, dec1, id, x0 + lx, y0 + ly, z0 + lz + 1);
                         }
                     });
             };
@@ -245,8 +231,7 @@ __global__ void __launch_bounds__(kDepThreads, Policy::kCtas) deposit_block_kern
     }
     float p0, p1;
     unpk(poison, p0, p1);
-    over = over || !(p0 == p0) || !(p1 == p1);
-    if (over && !D.emit_only) atomicOr(err, 4);
+    if ((!(p0 == p0) || !(p1 == p1)) && !D.emit_only) atomicOr(err, 4);
     nacc = __reduce_add_sync(0xffffffffu, nacc);   // a tile's pairs: at most 2^26 records x 1024 points / 8 warps
     if (lane == 0 && tally && !D.emit_only && nacc) atomicAdd(tally, (unsigned long long)nacc);
     __syncthreads();

@@ -737,8 +737,10 @@ int launch_piece(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out);
 int launch_scatter(Ctx *c, const CenterlineBatch &B);
 
 // Lines whose truncation radius Rtube_ratio * sigma_max is at most this many grid spacings go
-// through the piece kernel; thicker tubes through the sub-segment kernel, whose analytic
-// row intervals skip most of a large box.
+// through the piece kernels; thicker tubes through the sub-segment kernels.  (At 6.5 and 7.6
+// spacings the block kernel would be 1.05 and 1.3 times as fast, but it tests a point's distance
+// to the chord from the sub-segment's own frame: points within rounding of Rtube, where the
+// truncated profile steps by up to 4e-4 of its peak, would fall on the other side.)
 constexpr double kPieceMaxRtCells = 8.0;
 // Piece lines whose truncation radius is at most this many grid spacings can have their pieces
 // rasterised once (piece_raster) instead of searched in every tile.  Off by default: on the
@@ -752,5 +754,9 @@ constexpr double kRasterMaxRtCells = 0.0;
 // 1024^3 workload the scatter path took 0.34x (radius 1.9 grid spacings) and 0.75x (3.8) of the
 // tile path's deposition time, and 1.5x at 7.6, where a chord accepts hundreds of points.
 constexpr double kScatterMaxRtCells = 5.0;
+// With a constant core the tile-free path is the faster one up to the piece limit (512^3, 512
+// tubes of 4096 nodes, ms against the piece tile kernel: 5.5: 114 / 135, 6.5: 189 / 205, 7.6:
+// 308 / 306).
+constexpr double kScatterMaxRtCellsConst = 8.0;
 
 }  // namespace fwt

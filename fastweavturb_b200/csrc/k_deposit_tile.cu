@@ -546,7 +546,7 @@ struct SegBlocks {
                    : kBoxed;
     }
     // The lane's two points, (lx, ly, lz) and (lx, ly, lz + 1) in the tile.
-    template <bool General, int Form, typename Sink>
+    template <int Form, typename Sink>
     static __device__ __forceinline__ void visit(const Prep &P, const SegRec &R, int k, float dx, float lx, float ly,
                                                  float lz, bool in0, bool in1, Sink &&sink)
     {
@@ -577,11 +577,10 @@ struct SegBlocks {
         }
         const bool sure0 = ma >= pe, sure1 = mb >= pe;
         f32x2 v[3];
-        float cond0 = 1.0f, cond1 = 1.0f;
-        if constexpr (General || Form == kWrapped) {
-            float a[3], b[3];
-            rec_vorticity<General, Form == kWrapped>(R, x, y, za, ta, a, cond0);
-            rec_vorticity<General, Form == kWrapped>(R, x, y, zb, tb, b, cond1);
+        if constexpr (Form == kWrapped) {
+            float a[3], b[3], cond;
+            rec_vorticity<false>(R, x, y, za, ta, a, cond);
+            rec_vorticity<false>(R, x, y, zb, tb, b, cond);
 #pragma unroll
             for (int d = 0; d < 3; ++d) v[d] = pk(a[d], b[d]);
         } else {
@@ -613,7 +612,7 @@ struct SegBlocks {
 #pragma unroll
             for (int d = 0; d < 3; ++d) v[d] = mul2(tp, mul2(c1[d], in1_));
         }
-        sink(ok0 && sure0, ok1 && sure1, ok0 && !sure0, ok1 && !sure1, 0, 0, v, cond0, cond1);
+        sink(ok0 && sure0, ok1 && sure1, ok0 && !sure0, ok1 && !sure1, v);
     }
 };
 
@@ -884,11 +883,11 @@ int launch_tile(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
     } while (0)
         const unsigned grid = (unsigned)(std::min<int64_t>(ntiles, L.w1) - L.w0);
         const int m = kt_begin(c, KT_DEPOSIT);
-#define FWT_BLOCK_LAUNCH(G, A)                                                                             \
+#define FWT_BLOCK_LAUNCH(A)                                                                             \
     do {                                                                                                   \
-        FWT_CUDA(cudaFuncSetAttribute(deposit_block_kernel<SegBlocks, G, A>,                               \
+        FWT_CUDA(cudaFuncSetAttribute(deposit_block_kernel<SegBlocks, A>,                               \
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem<SegBlocks>())); \
-        deposit_block_kernel<SegBlocks, G, A><<<grid * parts, kDepThreads, block_smem<SegBlocks>(), c->stream>>>( \
+        deposit_block_kernel<SegBlocks, A><<<grid * parts, kDepThreads, block_smem<SegBlocks>(), c->stream>>>( \
             B.rec, N, ntx, nty, tz0, (int)parts, d_toff, d_list, scale, (float *)wx, (float *)wy, (float *)wz, d_err, \
             rctx.zs, rctx.zs + rctx.nz, (float)dxg, rctx.tally, L);                                       \
         FWT_CUDA(cudaGetLastError());                                                                      \
@@ -897,9 +896,9 @@ int launch_tile(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
             // the FP64 path evaluates every pair in FP64: the General distinction is only the FP32 one
             if (accumulate) FWT_TILE_LAUNCH(true, true, true); else FWT_TILE_LAUNCH(true, false, true);
         } else if (general) {
-            if (accumulate) FWT_BLOCK_LAUNCH(true, true); else FWT_BLOCK_LAUNCH(true, false);
+            if (accumulate) FWT_TILE_LAUNCH(true, true, false); else FWT_TILE_LAUNCH(true, false, false);
         } else {
-            if (accumulate) FWT_BLOCK_LAUNCH(false, true); else FWT_BLOCK_LAUNCH(false, false);
+            if (accumulate) FWT_BLOCK_LAUNCH(true); else FWT_BLOCK_LAUNCH(false);
         }
 #undef FWT_BLOCK_LAUNCH
 #undef FWT_TILE_LAUNCH

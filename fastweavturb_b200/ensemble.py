@@ -40,7 +40,7 @@ from .configs import build_workload
 TUNE_CANDIDATES = (0.0, 2.5, 5.0, 8.0)          # chord-piece kernel radius limit
 SCATTER_CANDIDATES = (0.0, 2.5, 5.0, 8.0)       # scatter kernel (no tiles) radius limit
 RASTER_CANDIDATES = (0.0, 1.5, 2.5, 4.0)        # rasterised pieces radius limit
-DEFAULTS = (8.0, 5.0, 0.0)                      # the library's defaults of the three limits
+DEFAULTS = (8.0, 8.0, 0.0)                      # the library's defaults of the three limits (constant core)
 
 
 class Ensemble:
