@@ -1,30 +1,42 @@
 // k_mlp.cu -- the learned surrogate: a multilayer perceptron n_in -> width x depth (GELU) ->
-// n_out whose matrix products run on the tensor cores (gemm_bf16_tc: BF16 operands, FP32
-// accumulation) and whose bias, activation, loss and Adam steps are FP32 elementwise kernels.
-// FP32 master weights; BF16 copies (and transposes, for the backward products) are refreshed
-// after every update.  No reference counterpart: the surrogate maps generator parameters to
-// the statistics the generator produces (the reference only plots those statistics).
+// n_out whose matrix products run on the tensor cores (BF16 operands, FP32 accumulation), with
+// the bias, activation, loss and activation gradient of each product in its epilogue.  FP32
+// master weights; BF16 copies (and transposes, for the backward products) are refreshed with
+// every update.  No reference counterpart: the surrogate maps generator parameters to the
+// statistics the generator produces (the reference only plots those statistics).
 //
 // Shapes (B = batch padded to a multiple of 64, Kl = layer input width padded to 64):
 //   forward   Z_l[B x N_l]  = H_{l-1}[B x K_l] . W_l[N_l x K_l]^T + b_l,  H_l = gelu(Z_l)
-//   backward  dW_l[N_l x K_l] = dZ_l^T[N_l x B] . (H_{l-1}^T[K_l x B])^T
-//             dH_{l-1}[B x K_l] = dZ_l[B x Np_l] . (W_l^T[K_l x Np_l])^T,  dZ = dH * gelu'(Z)
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-
+//   backward  dH_{l-1}[B x K_l] = dZ_l[B x Np_l] . (W_l^T[K_l x Np_l])^T,  dZ = dH * gelu'(Z)
+//             dW_l[N_l x K_l] = dZ_l^T[N_l x B] . (H_{l-1}^T[K_l x B])^T
+//
+// What bounds it: latency.  At the surrogate's batch of 256 a product is 34 MFLOP, under a
+// microsecond of one SM's tensor core, so a step is a chain of dependent launches.  The chain is
+// kept short -- pack, one launch per layer forward and back, one for all weight gradients, one for
+// the bias gradients, one for Adam and the BF16 copies: 13 launches for depth 4, against 57 with
+// the elementwise passes apart (one thread per column summed the bias gradients row by row) --
+// and each launch lets the next one start its prologue early (programmatic dependent launch):
+// barriers, tensor memory and the weights' tiles, which no kernel of the chain writes, are ready
+// when the previous product ends.  Inputs and results cross to the host in one copy each.
+// Batch 256, depth 4: 160 us a training step, 760 before; the input gradient of 192 rows 119 us, 628
+// before (about 8 us a layer: the wait for the product before, one load latency, the epilogue).
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <string>
 #include <vector>
 
 #include "../../include/fwt.h"
 #include "fwt_internal.h"
+#include "k_gemm_tc.cuh"
 
 namespace fwt {
 
 int gemm_bf16_tc(const void *A, const void *B, float *C, int M, int N, int K, int ldc, int *d_err, cudaStream_t st);
 
 static inline int pad64(int x) { return (x + 63) / 64 * 64; }
+static inline unsigned nblk(int64_t n) { return (unsigned)((n + 255) / 256); }
 
 struct MlpLayer {
     int K = 0, Kp = 0, N = 0, Np = 0;   // input/output widths and their 64-padded sizes
@@ -33,7 +45,7 @@ struct MlpLayer {
     float *gW = nullptr, *gb = nullptr;
     __nv_bfloat16 *Wh = nullptr;        // N x Kp
     __nv_bfloat16 *Wt = nullptr;        // Kp x Np (transpose)
-    float *Z = nullptr;                 // B x N pre-activation
+    float *Z = nullptr;                 // B x N pre-activation (hidden layers)
     __nv_bfloat16 *H = nullptr;         // B x Np activation (input of the next layer)
     __nv_bfloat16 *Ht = nullptr;        // Np x B
     float *dZf = nullptr;               // B x N
@@ -48,14 +60,21 @@ struct fwt_mlp {
     int n_in = 0, width = 0, depth = 0, n_out = 0, bmax = 0;
     std::vector<fwt::MlpLayer> L;
     __nv_bfloat16 *X0 = nullptr, *X0t = nullptr;   // B x 64, 64 x B
-    float *C = nullptr;                            // GEMM output scratch (max B x 256, 256 x 256)
-    float *T = nullptr, *wout = nullptr;           // targets B x n_out, output weights n_out
-    float *Xin = nullptr, *Gx = nullptr;           // inputs and input gradient, B x n_in
-    double *loss = nullptr;
-    int *err = nullptr;
+    // One exchange buffer with the host, and its mirror there: the loss (FP64), the error flag and a
+    // pad, then x (B x n_in; the input gradient replaces it), then the targets (B x n_out; the
+    // forward pass writes its outputs there), then the output weights (n_out).
+    // The mirror is ordinary memory: pinning it cost 14-25 ms a network and saved nothing measurable a step.
+    unsigned char *io = nullptr;
+    std::vector<unsigned char> hmem;
+    unsigned char *hio = nullptr;
     int64_t step = 0;
     cudaStream_t st = nullptr;
     std::vector<void *> allocs;
+
+    int *err() const { return (int *)(io + 8); }
+    float *x() const { return (float *)(io + 16); }
+    float *t(int B) const { return x() + (size_t)B * n_in; }
+    float *w(int B) const { return t(B) + (size_t)B * n_out; }
 };
 
 namespace fwt {
@@ -80,10 +99,14 @@ __device__ __forceinline__ float gelu_d(float x)
     return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
 
+constexpr size_t kIoHead = 16;   // bytes of the exchange buffer before x
+
 // X (B x n_in, FP32) -> X0 (Bp x 64 BF16, zero padded) and its transpose
 __global__ void mlp_pack_input(const float *__restrict__ X, int B, int Bp, int n_in, __nv_bfloat16 *__restrict__ X0,
                                __nv_bfloat16 *__restrict__ X0t)
 {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= Bp * 64) return;
     const int r = i / 64, c = i % 64;
@@ -93,99 +116,319 @@ __global__ void mlp_pack_input(const float *__restrict__ X, int B, int Bp, int n
     X0t[(size_t)c * Bp + r] = h;
 }
 
-// Z = C + b; hidden layers also H = gelu(Z) (BF16, zero padded to Np) and H^T
-__global__ void mlp_bias_act(const float *__restrict__ C, const float *__restrict__ b, int B, int Bp, int N, int Np,
-                             int act, float *__restrict__ Z, __nv_bfloat16 *__restrict__ H,
-                             __nv_bfloat16 *__restrict__ Ht)
+// What a product's epilogue does with element (r, c) of A . B^T:
+enum MlpEpi {
+    kHidden = 0,   // Z = . + b; H = gelu(Z) (BF16, zero padded to Np) and H^T
+    kOutput,       // Z = . + b
+    kLoss,         // y = . + b against the targets: loss = sum w (y - t)^2 / (B n), dZ of the output layer
+    kActBack,      // dZ = . * gelu'(Z) for a hidden layer
+    kWeight,       // the weight gradient, K wide
+    kInput         // the input gradient, n_in wide
+};
+
+struct MlpJob {
+    const __nv_bfloat16 *A, *Bm;   // M x K, Nb x K (rows beyond Nb count as zero)
+    int M, N, K, Nb;
+    int epi, b_const;              // b_const: B is not written by the kernels of this step
+    int B, Bp, Nl, Np;             // batch, padded batch, the output's width and its padded width
+    const float *bias;
+    float *Z;                      // B x Nl: written (kHidden, kOutput), read (kActBack)
+    __nv_bfloat16 *H, *Ht;         // Bp x Np and Np x Bp (kHidden); dZ and dZ^T (kLoss, kActBack)
+    float *F;                      // dZf (kLoss, kActBack), dW (kWeight), dX (kInput)
+    const float *T, *w;            // targets and output weights (kLoss)
+    double *loss;
+};
+
+constexpr int kMlpJobs = 8;       // products of one launch
+struct MlpJobs {
+    MlpJob j[kMlpJobs];
+};
+
+constexpr int kMlpBN = 32, kMlpStages = 4, kMlpThreads = 256;
+constexpr size_t kMlpStage = (size_t)(kGemmBM + kMlpBN) * kGemmBK * 2;
+constexpr size_t kMlpSmem = kMlpStage * kMlpStages;
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool in)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Bp * Np) return;
-    const int r = i / Np, c = i % Np;
-    float z = 0.0f;
-    if (r < B && c < N) {
-        z = C[(size_t)r * N + c] + b[c];
-        Z[(size_t)r * N + c] = z;
-    }
-    if (act) {
-        const float h = (r < B && c < N) ? gelu(z) : 0.0f;
-        const __nv_bfloat16 hb = __float2bfloat16_rn(h);
-        H[(size_t)r * Np + c] = hb;
-        Ht[(size_t)c * Bp + r] = hb;
-    }
+    const int n = in ? 16 : 0;   // rows beyond the matrix read zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 
-// loss = sum_b sum_j w_j (y - t)^2 / (B n_out); dZ of the output layer
-__global__ void mlp_loss_grad(const float *__restrict__ Y, const float *__restrict__ T, const float *__restrict__ w,
-                              int B, int Bp, int N, int Np, double *__restrict__ loss, float *__restrict__ dZf,
-                              __nv_bfloat16 *__restrict__ dZ, __nv_bfloat16 *__restrict__ dZt)
+// One 128 x 32 tile of job blockIdx.z per CTA: K in chunks of 64 through a ring of four stages (the
+// surrogate's K of 256 is staged whole), cp.async into the no-swizzle K-major layout, four
+// tcgen05.mma (M 128, N 32, K 16) per chunk into tensor memory, and the epilogue by eight warps
+// (16 columns each) straight from it.  32 columns rather than 256: a layer of 256 x 256 at batch
+// 256 spreads over 16 SMs and the epilogue, the longest part, is an eighth as long.  Every wait is
+// bounded; on a timeout the CTA sets *err, still frees its tensor memory and returns.
+__global__ void __launch_bounds__(kMlpThreads) mlp_gemm_kernel(const __grid_constant__ MlpJobs jobs, int *__restrict__ err)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double l = 0.0;
-    if (i < Bp * Np) {
-        const int r = i / Np, c = i % Np;
-        float g = 0.0f;
-        if (r < B && c < N) {
-            const float d = Y[(size_t)r * N + c] - T[(size_t)r * N + c];
-            const float wc = w ? w[c] : 1.0f;
-            l = (double)wc * d * d / ((double)B * N);
-            g = 2.0f * wc * d / ((float)B * (float)N);
-            dZf[(size_t)r * N + c] = g;
+    const MlpJob &J = jobs.j[blockIdx.z];
+    const int m0 = blockIdx.x * kGemmBM, n0 = blockIdx.y * kMlpBN;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (m0 >= J.M || n0 >= J.N) {
+        // the next kernel may rely on this one's wait for all that came before
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        return;
+    }
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ uint64_t bar[kMlpStages];
+    __shared__ uint32_t tmem_base;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(smem);
+    const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(bar);
+    const int K = J.K, nk = K / kGemmBK;
+    auto load_a = [&](int kc) {
+        const uint32_t s = s0 + (uint32_t)(kc % kMlpStages) * (uint32_t)kMlpStage;
+        for (int i = tid; i < kGemmBM * 8; i += kMlpThreads) {
+            const int r = i >> 3, k8 = i & 7;
+            const bool in = m0 + r < J.M;
+            cp_async16(s + core_off(r, k8, kGemmBM), J.A + (size_t)(in ? m0 + r : 0) * K + kc * kGemmBK + k8 * 8, in);
         }
-        const __nv_bfloat16 gb = __float2bfloat16_rn(g);
-        dZ[(size_t)r * Np + c] = gb;
-        if (c < N) dZt[(size_t)c * Bp + r] = gb;
+    };
+    auto load_b = [&](int kc) {
+        const uint32_t s = s0 + (uint32_t)(kc % kMlpStages) * (uint32_t)kMlpStage + kGemmBM * kGemmBK * 2;
+        for (int i = tid; i < kMlpBN * 8; i += kMlpThreads) {
+            const int r = i >> 3, k8 = i & 7;
+            const bool in = n0 + r < J.Nb;
+            cp_async16(s + core_off(r, k8, kMlpBN), J.Bm + (size_t)(in ? n0 + r : 0) * K + kc * kGemmBK + k8 * 8, in);
+        }
+    };
+    if (warp == 0) {
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&tmem_base);
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "r"(kMlpBN));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
+    if (tid < kMlpStages)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8u * (uint32_t)tid) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    const int pre = min(nk, kMlpStages);
+    if (J.b_const)
+        for (int kc = 0; kc < pre; ++kc) load_b(kc);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int kc = 0; kc < kMlpStages; ++kc) {   // one group per stage, empty ones included
+        if (kc < pre) {
+            if (!J.b_const) load_b(kc);
+            load_a(kc);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_base;
+    const uint32_t idesc = umma_idesc_bf16(kGemmBM, kMlpBN);
+    // The epilogue's own operands, read while the product runs: warps w and w + 4 take accumulator
+    // lanes 32 (w & 3) .. + 31, 16 columns each.
+    const int row = m0 + (warp & 3) * 32 + lane, c0 = n0 + 16 * (warp >> 2);
+    const bool in_b = row < (J.epi == kWeight ? J.M : J.B);
+    const int nc = in_b ? max(0, min(16, J.Nl - c0)) : 0;   // this thread's columns inside the result
+    const size_t at = (size_t)row * J.Nl + c0;
+    const bool vec = nc == 16 && (J.Nl & 3) == 0;           // its 16 values start on 16 bytes
+    float e0[16], e1[16], e2[16];   // bias or Z; targets; output weights
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0 && l != 0.0) atomicAdd(loss, l);
-}
-
-// dZ = dH * gelu'(Z) for a hidden layer (dH = C, B x ldc)
-__global__ void mlp_act_back(const float *__restrict__ C, int ldc, const float *__restrict__ Z, int B, int Bp, int N,
-                             int Np, float *__restrict__ dZf, __nv_bfloat16 *__restrict__ dZ,
-                             __nv_bfloat16 *__restrict__ dZt)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Bp * Np) return;
-    const int r = i / Np, c = i % Np;
-    float g = 0.0f;
-    if (r < B && c < N) {
-        g = C[(size_t)r * ldc + c] * gelu_d(Z[(size_t)r * N + c]);
-        dZf[(size_t)r * N + c] = g;
+    for (int i = 0; i < 16; ++i) e0[i] = e1[i] = e2[i] = 0.0f;
+    if (J.epi == kActBack) {
+        if (vec) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<float4 *>(e0 + 4 * i) = *reinterpret_cast<const float4 *>(J.Z + at + 4 * i);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (i < nc) e0[i] = J.Z[at + i];
+        }
+    } else if (J.epi <= kLoss) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (i < nc) e0[i] = J.bias[c0 + i];
+        if (J.epi == kLoss) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (i < nc) {
+                    e1[i] = J.T[at + i];
+                    e2[i] = J.w[c0 + i];
+                }
+        }
     }
-    const __nv_bfloat16 gb = __float2bfloat16_rn(g);
-    dZ[(size_t)r * Np + c] = gb;
-    if (c < N) dZt[(size_t)c * Bp + r] = gb;
+    bool ok = true;
+    for (int kc = 0; kc < nk && ok; ++kc) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kMlpStages - 1) : "memory");
+        // the MMA reads shared memory through the async proxy
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (tid == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t sa = s0 + (uint32_t)(kc % kMlpStages) * (uint32_t)kMlpStage, sb = sa + kGemmBM * kGemmBK * 2;
+#pragma unroll
+            for (int kk = 0; kk < kGemmBK / 16; ++kk) {
+                // K = 16 covers the core matrices 2kk and 2kk+1 along K
+                const uint64_t da = umma_smem_desc(sa + (uint32_t)(2 * kk * kGemmBM * 16), kGemmBM * 16, 128);
+                const uint64_t db = umma_smem_desc(sb + (uint32_t)(2 * kk * kMlpBN * 16), kMlpBN * 16, 128);
+                const uint32_t acc = (kc > 0 || kk > 0) ? 1u : 0u;
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
+                    "l"(da), "l"(db), "r"(idesc), "r"(acc));
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             bar0 + 8u * (uint32_t)(kc % kMlpStages))
+                         : "memory");
+        }
+        // refill the stage of the chunk before, once its products have read it
+        const int nx = kc - 1 + kMlpStages;
+        if (kc > 0 && nx < nk) {
+            ok = gemm_mbar_wait(bar0 + 8u * (uint32_t)((kc - 1) % kMlpStages), (uint32_t)((kc - 1) / kMlpStages) & 1u);
+            ok = __syncthreads_and(ok) != 0;
+            if (ok) {
+                load_b(nx);
+                load_a(nx);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    if (ok) {
+        ok = gemm_mbar_wait(bar0 + 8u * (uint32_t)((nk - 1) % kMlpStages), (uint32_t)((nk - 1) / kMlpStages) & 1u);
+        ok = __syncthreads_and(ok) != 0;
+    }
+    if (!ok) {
+        if (tid == 0) atomicOr(err, 1);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        float v[16];
+        {
+            uint32_t u[16];
+            const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(16 * (warp >> 2));
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                "%14, %15}, [%16];"
+                : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]),
+                  "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+                : "r"(taddr));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(u[i]);
+        }
+        double l = 0.0;
+        float *keep = J.F;   // the FP32 values kept: B x Nl (kWeight: M x Nl)
+        if (J.epi <= kOutput) {
+            keep = J.Z;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] += e0[i];
+        } else if (J.epi == kActBack) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = v[i] * gelu_d(e0[i]);
+        } else if (J.epi == kLoss) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float d = (v[i] + e0[i]) - e1[i];
+                if (i < nc) l += (double)e2[i] * d * d / ((double)J.B * J.Nl);
+                v[i] = 2.0f * e2[i] * d / ((float)J.B * (float)J.Nl);
+            }
+        }
+        if (vec) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<float4 *>(keep + at + 4 * i) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (i < nc) keep[at + i] = v[i];
+        }
+        if (row < J.M && (J.epi == kHidden || J.epi == kLoss || J.epi == kActBack)) {
+            // a BF16 matrix for the next product, zero padded, and its transpose
+            __align__(16) __nv_bfloat16 h[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float o = J.epi == kHidden ? gelu(v[i]) : v[i];
+                h[i] = __float2bfloat16_rn(i < nc ? o : 0.0f);
+            }
+            if (c0 < J.Np) {   // Np is a multiple of 64: all 16 columns are inside or none
+                uint4 *out = reinterpret_cast<uint4 *>(J.H + (size_t)row * J.Np + c0);
+                out[0] = *reinterpret_cast<const uint4 *>(h);
+                out[1] = *reinterpret_cast<const uint4 *>(h + 8);
+            }
+            const int nt = (J.epi == kHidden ? J.Np : J.Nl) - c0;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (i < nt) J.Ht[(size_t)(c0 + i) * J.Bp + row] = h[i];
+        }
+        if (J.epi == kLoss) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+            if (lane == 0 && l != 0.0) atomicAdd(J.loss, l);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kMlpBN));
 }
 
-// db = column sums of dZ (FP32), one thread per column
-__global__ void mlp_bias_grad(const float *__restrict__ dZf, int B, int N, float *__restrict__ gb)
+// Per-layer arguments of the bias gradients and of Adam.
+struct MlpParam {
+    float *W, *mW, *vW, *gW, *b, *mb, *vb, *gb;
+    __nv_bfloat16 *Wh, *Wt;
+    const float *dZf;
+    int N, K, Kp, Np;
+};
+struct MlpParams {
+    MlpParam l[kMlpJobs];
+};
+
+// db = column sums of dZ (FP64 sums, fixed order): a block takes 32 columns of layer blockIdx.y, a
+// warp every eighth row.
+__global__ void __launch_bounds__(256) mlp_bias_grad(const __grid_constant__ MlpParams P, int B)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= N) return;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const MlpParam &L = P.l[blockIdx.y];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+    __shared__ double part[8][32];
     double s = 0.0;
-    for (int r = 0; r < B; ++r) s += dZf[(size_t)r * N + c];
-    gb[c] = (float)s;
+    if (c < L.N) {
+#pragma unroll 4
+        for (int r = warp; r < B; r += 8) s += L.dZf[(size_t)r * L.N + c];
+    }
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && c < L.N) {
+        double t = 0.0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t += part[i][lane];
+        L.gb[c] = (float)t;
+    }
 }
 
-// copy the GEMM's dW (N x Kp) into the K-wide gradient
-__global__ void mlp_take_grad(const float *__restrict__ C, int N, int K, int Kp, float *__restrict__ g)
+__device__ __forceinline__ float adam_step(float *p, const float *g, float *m1, float *m2, int i, float lr, float b1,
+                                           float b2, float c1, float c2, float eps)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N * K) return;
-    g[i] = C[(size_t)(i / K) * Kp + i % K];
-}
-
-__global__ void mlp_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m1,
-                         float *__restrict__ m2, int n, float lr, float b1, float b2, float c1, float c2, float eps)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
     const float gi = g[i];
     const float a = b1 * m1[i] + (1.0f - b1) * gi, v = b2 * m2[i] + (1.0f - b2) * gi * gi;
     m1[i] = a;
     m2[i] = v;
-    p[i] -= lr * (a / c1) / (sqrtf(v / c2) + eps);
+    const float q = p[i] - lr * (a / c1) / (sqrtf(v / c2) + eps);
+    p[i] = q;
+    return q;
+}
+
+// Adam on every weight and bias of the layers, and the weights' BF16 copies; nothing when a product
+// of the step timed out (*err).
+__global__ void __launch_bounds__(256) mlp_adam(const __grid_constant__ MlpParams P, float lr, float b1, float b2, float c1,
+                                                float c2, float eps, const int *__restrict__ err)
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const MlpParam &L = P.l[blockIdx.y];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, n = L.N * L.K;
+    if (*err != 0) return;
+    if (i < n) {
+        const __nv_bfloat16 h =
+            __float2bfloat16_rn(adam_step(L.W, L.gW, L.mW, L.vW, i, lr, b1, b2, c1, c2, eps));
+        const int r = i / L.K, k = i % L.K;
+        L.Wh[(size_t)r * L.Kp + k] = h;
+        L.Wt[(size_t)k * L.Np + r] = h;
+    } else if (i < n + L.N) {
+        adam_step(L.b, L.gb, L.mb, L.vb, i - n, lr, b1, b2, c1, c2, eps);
+    }
 }
 
 // BF16 copies of W: Wh (N x Kp, zero padded) and Wt (Kp x Np)
@@ -200,8 +443,6 @@ __global__ void mlp_refresh(const float *__restrict__ W, int N, int K, int Kp, i
     Wt[(size_t)k * Np + n] = v;
 }
 
-static inline unsigned nblk(int64_t n) { return (unsigned)((n + 255) / 256); }
-
 static int mlp_refresh_all(fwt_mlp *m)
 {
     for (auto &l : m->L)
@@ -210,61 +451,188 @@ static int mlp_refresh_all(fwt_mlp *m)
     return 0;
 }
 
-static int mlp_forward(fwt_mlp *m, const float *dX, int B)
+// Launch with the programmatic dependence on the kernel before it in the stream (every kernel of the
+// chain waits for it with griddepcontrol.wait before it touches what that kernel writes).
+template <typename K, typename... Args>
+static int mlp_launch(fwt_mlp *m, K kernel, dim3 grid, int threads, size_t smem, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = m->st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FWT_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+    return 0;
+}
+
+static int mlp_products(fwt_mlp *m, const MlpJob *j, int n)
+{
+    for (int o = 0; o < n; o += kMlpJobs) {
+        MlpJobs jobs = {};
+        int M = 0, N = 0;
+        const int c = std::min(kMlpJobs, n - o);
+        for (int i = 0; i < c; ++i) {
+            jobs.j[i] = j[o + i];
+            M = std::max(M, j[o + i].M);
+            N = std::max(N, j[o + i].N);
+        }
+        const dim3 grid((unsigned)((M + kGemmBM - 1) / kGemmBM), (unsigned)((N + kMlpBN - 1) / kMlpBN), (unsigned)c);
+        FWT_TRY(mlp_launch(m, mlp_gemm_kernel, grid, kMlpThreads, kMlpSmem, jobs, m->err()));
+    }
+    return 0;
+}
+
+// Forward pass of the batch in the exchange buffer; the output layer's values go to the targets'
+// place, or (loss) to the loss and its gradient.
+static int mlp_forward(fwt_mlp *m, int B, bool loss)
 {
     const int Bp = pad64(B);
-    mlp_pack_input<<<nblk((int64_t)Bp * 64), 256, 0, m->st>>>(dX, B, Bp, m->n_in, m->X0, m->X0t);
+    FWT_TRY(mlp_launch(m, mlp_pack_input, dim3(nblk((int64_t)Bp * 64)), 256, 0, (const float *)m->x(), B, Bp, m->n_in, m->X0,
+                       m->X0t));
     const __nv_bfloat16 *Hin = m->X0;
     for (size_t li = 0; li < m->L.size(); ++li) {
         MlpLayer &l = m->L[li];
-        FWT_TRY(gemm_bf16_tc(Hin, l.Wh, m->C, Bp, l.N, l.Kp, l.N, m->err, m->st));
-        const int act = li + 1 < m->L.size() ? 1 : 0;
-        mlp_bias_act<<<nblk((int64_t)Bp * l.Np), 256, 0, m->st>>>(m->C, l.b, B, Bp, l.N, l.Np, act, l.Z, l.H, l.Ht);
+        const bool last = li + 1 == m->L.size();
+        MlpJob j = {};
+        j.A = Hin;
+        j.Bm = l.Wh;
+        j.M = Bp;
+        j.N = l.N;
+        j.Nb = l.N;
+        j.K = l.Kp;
+        j.b_const = 1;
+        j.B = B;
+        j.Bp = Bp;
+        j.Nl = l.N;
+        j.Np = l.Np;
+        j.bias = l.b;
+        if (!last) {
+            j.epi = kHidden;
+            j.N = l.Np;   // the padding of H is written too
+            j.Z = l.Z;
+            j.H = l.H;
+            j.Ht = l.Ht;
+        } else if (!loss) {
+            j.epi = kOutput;
+            j.Z = m->t(B);
+        } else {
+            j.epi = kLoss;
+            j.N = l.Np;
+            j.H = l.dZ;
+            j.Ht = l.dZt;
+            j.F = l.dZf;
+            j.T = m->t(B);
+            j.w = m->w(B);
+            j.loss = (double *)m->io;
+        }
+        FWT_TRY(mlp_products(m, &j, 1));
         Hin = l.H;
     }
-    FWT_CUDA(cudaGetLastError());
     return 0;
 }
 
-// gradients of the weighted MSE w.r.t. every parameter (into l.gW, l.gb) and, if dXout, the
-// inputs (B x n_in, device)
-static int mlp_backward(fwt_mlp *m, int B, float *dXout)
+static void mlp_param_list(fwt_mlp *m, size_t o, int c, MlpParams &P)
+{
+    P = {};
+    for (int i = 0; i < c; ++i) {
+        MlpLayer &l = m->L[o + i];
+        P.l[i] = {l.W, l.mW, l.vW, l.gW, l.b, l.mb, l.vb, l.gb, l.Wh, l.Wt, l.dZf, l.N, l.K, l.Kp, l.Np};
+    }
+}
+
+// After mlp_forward(loss): the gradients of the weighted MSE w.r.t. the inputs (in the inputs' place)
+// and, if params, every parameter (into l.gW, l.gb).
+static int mlp_backward(fwt_mlp *m, int B, bool params, bool inputs)
 {
     const int Bp = pad64(B);
-    FWT_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(double), m->st));
-    MlpLayer &o = m->L.back();
-    mlp_loss_grad<<<nblk((int64_t)Bp * o.Np), 256, 0, m->st>>>(o.Z, m->T, m->wout, B, Bp, o.N, o.Np, m->loss, o.dZf,
-                                                                 o.dZ, o.dZt);
-    for (int li = (int)m->L.size() - 1; li >= 0; --li) {
+    for (int li = (int)m->L.size() - 1; li > 0 || (li == 0 && inputs); --li) {
         MlpLayer &l = m->L[li];
-        const __nv_bfloat16 *Hprev_t = li > 0 ? m->L[li - 1].Ht : m->X0t;
-        // dW = dZ^T . Hprev   (M = N_l, N = Kp, K = Bp)
-        FWT_TRY(gemm_bf16_tc(l.dZt, Hprev_t, m->C, l.N, l.Kp, Bp, l.Kp, m->err, m->st));
-        mlp_take_grad<<<nblk((int64_t)l.N * l.K), 256, 0, m->st>>>(m->C, l.N, l.K, l.Kp, l.gW);
-        mlp_bias_grad<<<nblk(l.N), 256, 0, m->st>>>(l.dZf, B, l.N, l.gb);
-        if (li == 0 && !dXout) break;
         // dH_prev = dZ . W  (M = Bp, N = Kp, K = Np)
-        FWT_TRY(gemm_bf16_tc(l.dZ, l.Wt, m->C, Bp, l.Kp, l.Np, l.Kp, m->err, m->st));
+        MlpJob j = {};
+        j.A = l.dZ;
+        j.Bm = l.Wt;
+        j.M = Bp;
+        j.N = j.Nb = l.Kp;
+        j.K = l.Np;
+        j.b_const = 1;
+        j.B = B;
+        j.Bp = Bp;
         if (li == 0) {
-            // input gradient: the first n_in columns
-            FWT_CUDA(cudaMemcpy2DAsync(dXout, sizeof(float) * m->n_in, m->C, sizeof(float) * l.Kp,
-                                       sizeof(float) * m->n_in, B, cudaMemcpyDeviceToDevice, m->st));
-            break;
+            j.epi = kInput;
+            j.Nl = m->n_in;
+            j.F = m->x();
+        } else {
+            MlpLayer &p = m->L[li - 1];
+            j.epi = kActBack;
+            j.Nl = p.N;
+            j.Np = p.Np;
+            j.Z = p.Z;
+            j.H = p.dZ;
+            j.Ht = p.dZt;
+            j.F = p.dZf;
         }
-        MlpLayer &p = m->L[li - 1];
-        mlp_act_back<<<nblk((int64_t)Bp * p.Np), 256, 0, m->st>>>(m->C, l.Kp, p.Z, B, Bp, p.N, p.Np, p.dZf, p.dZ,
-                                                                    p.dZt);
+        FWT_TRY(mlp_products(m, &j, 1));
     }
-    FWT_CUDA(cudaGetLastError());
+    if (!params) return 0;
+    // dW = dZ^T . Hprev  (M = N_l, N = Kp, K = Bp), every layer in one launch
+    std::vector<MlpJob> jobs;
+    for (size_t li = 0; li < m->L.size(); ++li) {
+        MlpLayer &l = m->L[li];
+        MlpJob j = {};
+        j.A = l.dZt;
+        j.Bm = li > 0 ? m->L[li - 1].Ht : m->X0t;
+        j.M = l.N;
+        j.N = j.Nb = l.Kp;
+        j.K = Bp;
+        j.epi = kWeight;
+        j.B = B;
+        j.Nl = l.K;
+        j.F = l.gW;
+        jobs.push_back(j);
+    }
+    FWT_TRY(mlp_products(m, jobs.data(), (int)jobs.size()));
+    for (size_t o = 0; o < m->L.size(); o += kMlpJobs) {
+        const int c = (int)std::min<size_t>(kMlpJobs, m->L.size() - o);
+        MlpParams P;
+        mlp_param_list(m, o, c, P);
+        int N = 0;
+        for (int i = 0; i < c; ++i) N = std::max(N, P.l[i].N);
+        FWT_TRY(mlp_launch(m, mlp_bias_grad, dim3((unsigned)((N + 31) / 32), (unsigned)c), 256, 0, P, B));
+    }
     return 0;
 }
 
-static int mlp_check_err(fwt_mlp *m)
+// The inputs, targets and output weights (1 where w_out is null) of a batch to the device, with the
+// loss and the error flag zeroed: one copy.
+static int mlp_upload(fwt_mlp *m, const float *x, const float *t, const float *w_out, int B)
 {
-    int herr = 0;
-    FWT_CUDA(cudaMemcpyAsync(&herr, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->st));
+    std::memset(m->hio, 0, kIoHead);
+    float *h = (float *)(m->hio + kIoHead);
+    std::memcpy(h, x, sizeof(float) * (size_t)B * m->n_in);
+    size_t n = (size_t)B * m->n_in;
+    if (t) {
+        std::memcpy(h + n, t, sizeof(float) * (size_t)B * m->n_out);
+        n += (size_t)B * m->n_out;
+        for (int i = 0; i < m->n_out; ++i) h[n + i] = w_out ? w_out[i] : 1.0f;
+        n += m->n_out;
+    }
+    FWT_CUDA(cudaMemcpyAsync(m->io, m->hio, kIoHead + sizeof(float) * n, cudaMemcpyHostToDevice, m->st));
+    return 0;
+}
+
+// The head of the exchange buffer and `floats` values after it, in the mirror; waits.
+static int mlp_download(fwt_mlp *m, size_t floats)
+{
+    FWT_CUDA(cudaMemcpyAsync(m->hio, m->io, kIoHead + sizeof(float) * floats, cudaMemcpyDeviceToHost, m->st));
     FWT_CUDA(cudaStreamSynchronize(m->st));
-    if (herr) return fail(FWT_E_TIMEOUT, "mlp: tensor-core GEMM wait ran out");
+    int herr = 0;
+    std::memcpy(&herr, m->hio + 8, sizeof(int));
+    if (herr) return fail(FWT_E_TIMEOUT, "mlp: tensor-core product's wait ran out");
     return 0;
 }
 
@@ -354,18 +722,13 @@ int fwt_mlp_create(int device, int n_in, int width, int depth, int n_out, int ba
     }
     try_(mlp_alloc(m, &m->X0, (size_t)Bp * 64));
     try_(mlp_alloc(m, &m->X0t, (size_t)64 * Bp));
-    try_(mlp_alloc(m, &m->C, (size_t)std::max(Bp, 256) * 256));
-    try_(mlp_alloc(m, &m->T, (size_t)Bp * n_out));
-    try_(mlp_alloc(m, &m->Xin, (size_t)Bp * n_in));
-    try_(mlp_alloc(m, &m->Gx, (size_t)Bp * n_in));
-    try_(mlp_alloc(m, &m->wout, n_out));
-    try_(mlp_alloc(m, &m->loss, 1));
-    try_(mlp_alloc(m, &m->err, 1));
-    if (rc == 0) {
-        std::vector<float> ones(n_out, 1.0f);
-        cudaMemcpy(m->wout, ones.data(), sizeof(float) * n_out, cudaMemcpyHostToDevice);
-        rc = mlp_refresh_all(m);
-    }
+    const size_t io_bytes = kIoHead + sizeof(float) * ((size_t)Bp * (n_in + n_out) + n_out);
+    try_(mlp_alloc(m, &m->io, io_bytes));
+    m->hmem.resize(io_bytes);
+    m->hio = m->hmem.data();
+    if (rc == 0 && cudaFuncSetAttribute(mlp_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMlpSmem) != cudaSuccess)
+        rc = fail(FWT_E_CUDA, "mlp: kernel attribute");
+    if (rc == 0) rc = mlp_refresh_all(m);
     if (rc == 0 && cudaStreamSynchronize(m->st) != cudaSuccess) rc = fail(FWT_E_CUDA, "mlp: set-up failed");
     if (rc) {
         fwt_mlp_destroy(m);
@@ -430,12 +793,12 @@ int fwt_mlp_forward(fwt_mlp *m, const float *x, int batch, float *y)
 {
     if (!m || !x || !y || batch < 1 || batch > m->bmax) return fail(FWT_E_ARG, "mlp: batch outside 1..batch_max");
     cudaSetDevice(m->dev);
-    float *dX = m->Xin;
-    FWT_CUDA(cudaMemsetAsync(m->err, 0, sizeof(int), m->st));
-    FWT_CUDA(cudaMemcpyAsync(dX, x, sizeof(float) * batch * m->n_in, cudaMemcpyHostToDevice, m->st));
-    FWT_TRY(mlp_forward(m, dX, batch));
-    FWT_CUDA(cudaMemcpyAsync(y, m->L.back().Z, sizeof(float) * batch * m->n_out, cudaMemcpyDeviceToHost, m->st));
-    return mlp_check_err(m);
+    FWT_TRY(mlp_upload(m, x, nullptr, nullptr, batch));
+    FWT_TRY(mlp_forward(m, batch, false));
+    const size_t nx = (size_t)batch * m->n_in, ny = (size_t)batch * m->n_out;
+    FWT_TRY(mlp_download(m, nx + ny));
+    std::memcpy(y, m->hio + kIoHead + sizeof(float) * nx, sizeof(float) * ny);
+    return 0;
 }
 
 // loss and its gradients: grad_params (nparams, layout of fwt_mlp_get_params) and grad_x
@@ -445,46 +808,49 @@ int fwt_mlp_loss_grad(fwt_mlp *m, const float *x, const float *t, const float *w
 {
     if (!m || !x || !t || batch < 1 || batch > m->bmax) return fail(FWT_E_ARG, "mlp: batch outside 1..batch_max");
     cudaSetDevice(m->dev);
-    float *dX = m->Xin, *dGx = m->Gx;
-    FWT_CUDA(cudaMemsetAsync(m->err, 0, sizeof(int), m->st));
-    FWT_CUDA(cudaMemcpyAsync(dX, x, sizeof(float) * batch * m->n_in, cudaMemcpyHostToDevice, m->st));
-    FWT_CUDA(cudaMemcpyAsync(m->T, t, sizeof(float) * batch * m->n_out, cudaMemcpyHostToDevice, m->st));
-    std::vector<float> ones(m->n_out, 1.0f);
-    FWT_CUDA(cudaMemcpyAsync(m->wout, w_out ? w_out : ones.data(), sizeof(float) * m->n_out, cudaMemcpyHostToDevice,
-                             m->st));
-    int rc = mlp_forward(m, dX, batch);
-    if (rc == 0) rc = mlp_backward(m, batch, grad_x ? dGx : nullptr);
-    if (rc == 0 && loss) rc = cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->st) ? -2 : 0;
-    if (rc == 0 && grad_x)
-        rc = cudaMemcpyAsync(grad_x, dGx, sizeof(float) * batch * m->n_in, cudaMemcpyDeviceToHost, m->st) ? -2 : 0;
-    if (rc == 0 && grad_params) {
+    FWT_TRY(mlp_upload(m, x, t, w_out, batch));
+    FWT_TRY(mlp_forward(m, batch, true));
+    FWT_TRY(mlp_backward(m, batch, grad_params != nullptr, grad_x != nullptr));
+    if (grad_params) {
         float *h = grad_params;
         for (auto &l : m->L) {
-            cudaMemcpyAsync(h, l.gW, sizeof(float) * l.N * l.K, cudaMemcpyDeviceToHost, m->st);
+            FWT_CUDA(cudaMemcpyAsync(h, l.gW, sizeof(float) * l.N * l.K, cudaMemcpyDeviceToHost, m->st));
             h += (size_t)l.N * l.K;
-            cudaMemcpyAsync(h, l.gb, sizeof(float) * l.N, cudaMemcpyDeviceToHost, m->st);
+            FWT_CUDA(cudaMemcpyAsync(h, l.gb, sizeof(float) * l.N, cudaMemcpyDeviceToHost, m->st));
             h += l.N;
         }
     }
-    if (rc) return rc < -1 ? fail(FWT_E_CUDA, "mlp: copy failed") : rc;
-    return mlp_check_err(m);
+    const size_t nx = grad_x ? (size_t)batch * m->n_in : 0;
+    FWT_TRY(mlp_download(m, nx));
+    if (loss) std::memcpy(loss, m->hio, sizeof(double));
+    if (grad_x) std::memcpy(grad_x, m->hio + kIoHead, sizeof(float) * nx);
+    return 0;
 }
 
 // one Adam step (beta1 0.9, beta2 0.999, eps 1e-8) on the weighted MSE of a batch
 int fwt_mlp_train_step(fwt_mlp *m, const float *x, const float *t, const float *w_out, int batch, float lr,
                        double *loss)
 {
-    FWT_TRY(fwt_mlp_loss_grad(m, x, t, w_out, batch, loss, nullptr, nullptr));
-    m->step += 1;
+    if (!m || !x || !t || batch < 1 || batch > m->bmax) return fail(FWT_E_ARG, "mlp: batch outside 1..batch_max");
+    cudaSetDevice(m->dev);
+    FWT_TRY(mlp_upload(m, x, t, w_out, batch));
+    FWT_TRY(mlp_forward(m, batch, true));
+    FWT_TRY(mlp_backward(m, batch, true, false));
+    const int64_t step = m->step + 1;
     const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.0f - (float)std::pow(0.9, (double)m->step), c2 = 1.0f - (float)std::pow(0.999, (double)m->step);
-    for (auto &l : m->L) {
-        mlp_adam<<<nblk((int64_t)l.N * l.K), 256, 0, m->st>>>(l.W, l.gW, l.mW, l.vW, l.N * l.K, lr, b1, b2, c1, c2,
-                                                               1e-8f);
-        mlp_adam<<<nblk(l.N), 256, 0, m->st>>>(l.b, l.gb, l.mb, l.vb, l.N, lr, b1, b2, c1, c2, 1e-8f);
+    const float c1 = 1.0f - (float)std::pow(0.9, (double)step), c2 = 1.0f - (float)std::pow(0.999, (double)step);
+    for (size_t o = 0; o < m->L.size(); o += kMlpJobs) {
+        const int c = (int)std::min<size_t>(kMlpJobs, m->L.size() - o);
+        MlpParams P;
+        mlp_param_list(m, o, c, P);
+        int64_t n = 0;
+        for (int i = 0; i < c; ++i) n = std::max<int64_t>(n, (int64_t)P.l[i].N * P.l[i].K + P.l[i].N);
+        FWT_TRY(mlp_launch(m, mlp_adam, dim3(nblk(n), (unsigned)c), 256, 0, P, lr, b1, b2, c1, c2, 1e-8f,
+                           (const int *)m->err()));
     }
-    FWT_TRY(mlp_refresh_all(m));
-    FWT_CUDA(cudaStreamSynchronize(m->st));
+    FWT_TRY(mlp_download(m, 0));   // a step that timed out left the weights as they were
+    m->step = step;
+    if (loss) std::memcpy(loss, m->hio, sizeof(double));
     return 0;
 }
 
