@@ -1,7 +1,7 @@
 // k_stats.cu -- statistics of the woven field:
 //   minmax_kernel      component ranges, bit-exact (order-preserving integer atomics)
-//   pdf_kernel         REAL(4) bin search of subroutine.f90:22-34 as a binary search on
-//                      the bins' upper edges, integer shared-memory histograms
+//   pdf_kernel         REAL(4) bin search of subroutine.f90:22-34 from the bin size and the
+//                      edges beside the guess, integer shared-memory histograms
 //   sp_kernel          longitudinal increments at separations r, moments p = 1..pmax
 //                      accumulated in FP64 (subroutine.f90:64-129); lines staged in shared
 //                      memory so each velocity component is read from HBM once
@@ -12,20 +12,44 @@
 
 namespace fwt {
 
-// Component range, exact in the field's precision: FP32 values through order-preserving
-// 32-bit atomics, FP64 values through 64-bit ones (mm: two words of the value's width).
+// Component ranges, exact in the field's precision: FP32 values through order-preserving 32-bit
+// atomics, FP64 values through 64-bit ones (mm: two words of the value's width per component,
+// component blockIdx.y).  Bound by HBM: 16-byte loads, four of them in flight per thread.
 template <typename Real>
-__global__ void minmax_kernel(const Real *__restrict__ a, size_t n, void *__restrict__ mm)
+__global__ void __launch_bounds__(256) minmax_kernel(const Real *__restrict__ f, size_t n, void *__restrict__ mm)
 {
     Real mn = (Real)3.4e38f, mx = (Real)-3.4e38f;
     if (sizeof(Real) == 8) {
         mn = (Real)1.7e308;
         mx = (Real)-1.7e308;
     }
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const Real v = a[i];
-        mn = fmin(mn, v);
-        mx = fmax(mx, v);
+    constexpr int kV = 16 / sizeof(Real);
+    struct __align__(16) Vec {
+        Real v[kV];
+    };
+    const Real *a = f + blockIdx.y * n;   // n is a multiple of 8 (N is even): the components start on 16 bytes
+    const size_t nv = n / kV, step = (size_t)gridDim.x * blockDim.x;
+    const Vec *av = reinterpret_cast<const Vec *>(a);
+    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (; i + 3 * step < nv; i += 4 * step) {
+        Vec q[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = av[i + k * step];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int j = 0; j < kV; ++j) {
+                mn = fmin(mn, q[k].v[j]);
+                mx = fmax(mx, q[k].v[j]);
+            }
+    }
+    for (; i < nv; i += step) {
+        const Vec q = av[i];
+#pragma unroll
+        for (int j = 0; j < kV; ++j) {
+            mn = fmin(mn, q.v[j]);
+            mx = fmax(mx, q.v[j]);
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -34,22 +58,28 @@ __global__ void minmax_kernel(const Real *__restrict__ a, size_t n, void *__rest
     }
     if ((threadIdx.x & 31) == 0) {
         if constexpr (sizeof(Real) == 8) {
-            unsigned long long *m = (unsigned long long *)mm;
+            unsigned long long *m = (unsigned long long *)mm + 2 * blockIdx.y;
             atomicMin(m, d2ord((double)mn));
             atomicMax(m + 1, d2ord((double)mx));
         } else {
-            uint32_t *m = (uint32_t *)mm;
+            uint32_t *m = (uint32_t *)mm + 2 * blockIdx.y;
             atomicMin(m, f2ord((float)mn));
             atomicMax(m + 1, f2ord((float)mx));
         }
     }
 }
 
-// v = (float)((double)x * s); bin = first l with v < hi[l], counted if lo[l] <= v
+// Histogram of v = (float)((double)x * s) over n values: bin = first l with v < hi[l], counted if
+// lo[l] <= v.  The upper edges never decrease, so the bin is found from the guess (v - vmin) /
+// bin size and the edges beside it, instead of a binary search (eight dependent shared loads at
+// 201 bins).  The counts are kept in `copies` (a power of two up to 32) interleaved copies, lane
+// i in copy i mod copies: with 32 every lane has its own bank and a field whose values crowd into
+// one bin (omega between the tubes) costs no more than a flat one.  Six components of 512^3, 201
+// bins: 4.96 ms with the search and one copy, 1.75 now; reading them takes 0.5.
 template <typename Real>
-__global__ void __launch_bounds__(256) pdf_kernel(const Real *__restrict__ a, size_t n, double s,
+__global__ void __launch_bounds__(256) pdf_kernel(const Real *__restrict__ a, size_t n, double s, float vmin, float ibsz,
                                                   const float *__restrict__ lo, const float *__restrict__ hi, int nbins,
-                                                  unsigned long long *__restrict__ counts)
+                                                  int copies, unsigned long long *__restrict__ counts)
 {
     extern __shared__ unsigned char smem[];
     float *s_hi = (float *)smem;
@@ -58,115 +88,166 @@ __global__ void __launch_bounds__(256) pdf_kernel(const Real *__restrict__ a, si
     for (int i = threadIdx.x; i < nbins; i += blockDim.x) {
         s_hi[i] = hi[i];
         s_lo[i] = lo[i];
-        s_cnt[i] = 0;
+    }
+    for (int i = threadIdx.x; i < nbins * copies; i += blockDim.x) s_cnt[i] = 0;
+    __syncthreads();
+    const int mine = (int)threadIdx.x & (copies - 1);
+    const float last = s_hi[nbins - 1];
+    auto count = [&](Real x) {
+        const float v = (float)((double)x * s);
+        if (!(v < last)) return;   // beyond the last edge, or not a number
+        int l = min(max((int)((v - vmin) * ibsz), 0), nbins - 1);
+        while (l > 0 && v < s_hi[l - 1]) --l;
+        while (!(v < s_hi[l])) ++l;
+        if (s_lo[l] <= v) atomicAdd(s_cnt + l * copies + mine, 1u);
+    };
+    constexpr int kV = 16 / sizeof(Real);
+    struct __align__(16) Vec {
+        Real v[kV];
+    };
+    const size_t nv = n / kV, step = (size_t)gridDim.x * blockDim.x;   // n is a multiple of 8 (N is even)
+    const Vec *av = reinterpret_cast<const Vec *>(a);
+    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (; i + step < nv; i += 2 * step) {
+        const Vec p = av[i], q = av[i + step];
+#pragma unroll
+        for (int j = 0; j < kV; ++j) count(p.v[j]);
+#pragma unroll
+        for (int j = 0; j < kV; ++j) count(q.v[j]);
+    }
+    if (i < nv) {
+        const Vec p = av[i];
+#pragma unroll
+        for (int j = 0; j < kV; ++j) count(p.v[j]);
     }
     __syncthreads();
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float v = (float)((double)a[i] * s);
-        int lo_i = 0, hi_i = nbins;   // first l in [0, nbins) with v < s_hi[l]
-        while (lo_i < hi_i) {
-            const int mid = (lo_i + hi_i) >> 1;
-            if (v < s_hi[mid]) hi_i = mid;
-            else lo_i = mid + 1;
-        }
-        if (lo_i < nbins && s_lo[lo_i] <= v) atomicAdd(s_cnt + lo_i, 1u);
+    for (int i2 = threadIdx.x; i2 < nbins; i2 += blockDim.x) {
+        unsigned long long t = 0;
+        for (int k = 0; k < copies; ++k) t += s_cnt[i2 * copies + ((k + i2) & (copies - 1))];
+        if (t) atomicAdd(counts + i2, t);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nbins; i += blockDim.x)
-        if (s_cnt[i]) atomicAdd(counts + i, (unsigned long long)s_cnt[i]);
 }
 
 // Structure functions along one axis.  A block stages W lines of length N in shared memory
-// as [pos][line] (padded), in the field's own precision, then warp w accumulates, for its
-// separations, sum (du * s)^p for p = 1..PMAX in registers.  W = 32 lines for FP32 fields and
-// 16 for FP64 (a 1024-point FP64 group still fits one block's shared memory); groups at the end
-// of an axis may hold fewer lines, so any N works.  axis 0: u_x along x; 1: u_y along y;
-// 2: u_z along z.
+// as [pos][line] (padded), in the field's own precision; groups at the end of an axis may hold
+// fewer lines, so any N works.  axis 0: u_x along x; 1: u_y along y; 2: u_z along z.
+//
+// Bound by FP64 arithmetic: the sums of du^p, p = 1..PMAX, over every point and separation.  A
+// warp takes MPW separations and a share of the positions, so a point is read and widened once
+// for MPW increments; the sums use the even powers and fused multiply-adds (8 FP64 operations
+// for p <= 6, 14 for 10, where a running power took 21), the scale 1/u' enters as an exact power
+// of two when the lines are staged and as its remainder at the end, only as many orders as
+// asked for are summed, and separations equal modulo N once (the host's list).  512^3, three
+// components, orders 1-6: 14.5 ms with the running power to order 10, 7.8 now; at the FP64 rate
+// the 17 separations take 3.8.
 template <typename Real>
 __host__ __device__ constexpr int sp_lines(int N)
 {
     return N < (sizeof(Real) == 8 ? 16 : 32) ? N : (sizeof(Real) == 8 ? 16 : 32);
 }
+constexpr int kSpPerWarp = 4;   // separations of a warp
+constexpr int kSpGroups = 8, kSpMaxThreads = 384;   // groups of separations in a block; six of them twice
 
-// The field is a box n0 x n1 x n2 (x fastest) whose extent along `axis` is the line length N:
-// the whole grid, or a z-slab (axes 0, 1) or y-pencil (axis 2) of a grid split over GPUs.
-template <typename Real, int PMAX, int MPW>
-__global__ void __launch_bounds__(256) sp_kernel(const Real *__restrict__ u, int N, int n0, int n1, int n2, int axis,
-                                                 double s, const int *__restrict__ rs, int nr,
+template <int PMAX>
+__device__ __forceinline__ void sp_accumulate(double d, double (&acc)[PMAX])
+{
+    const double d2 = d * d;
+    acc[0] += d;
+    acc[1] += d2;
+    if (PMAX > 2) acc[2 < PMAX ? 2 : 0] = fma(d2, d, acc[2 < PMAX ? 2 : 0]);
+    if (PMAX > 3) {
+        const double d4 = d2 * d2;
+        acc[3 < PMAX ? 3 : 0] += d4;
+        if (PMAX > 4) acc[4 < PMAX ? 4 : 0] = fma(d4, d, acc[4 < PMAX ? 4 : 0]);
+        if (PMAX > 5) {
+            if (PMAX == 6) {
+                acc[5 < PMAX ? 5 : 0] = fma(d4, d2, acc[5 < PMAX ? 5 : 0]);
+            } else {
+                const double d6 = d4 * d2, d8 = d4 * d4;
+                acc[5 < PMAX ? 5 : 0] += d6;
+                acc[6 < PMAX ? 6 : 0] = fma(d6, d, acc[6 < PMAX ? 6 : 0]);
+                acc[7 < PMAX ? 7 : 0] += d8;
+                acc[8 < PMAX ? 8 : 0] = fma(d8, d, acc[8 < PMAX ? 8 : 0]);
+                acc[9 < PMAX ? 9 : 0] = fma(d8, d2, acc[9 < PMAX ? 9 : 0]);
+            }
+        }
+    }
+}
+
+// The field is a box n0 x n1 x n2 (x fastest) whose extent along the axis is the line length N:
+// the whole grid, or a z-slab (axes 0, 1) or y-pencil (axis 2) of a grid split over GPUs.  The
+// axis is axis0 + blockIdx.y, its component stride elements further on per step.  blockDim is
+// 32 x (groups of separations) x (1 or 2 shares of the positions).
+// Groups beyond eight go to blockIdx.z.
+template <typename Real, int PMAX>
+__global__ void __launch_bounds__(kSpMaxThreads, PMAX > 6 ? 1 : 2) sp_kernel(const Real *__restrict__ u0, size_t stride, int N, int n0, int n1, int n2,
+                                                 int axis0, Real sc, const int *__restrict__ rs, int nr,
                                                  double *__restrict__ Sp)
 {
     extern __shared__ __align__(16) unsigned char sp_smem[];
     Real *tile = reinterpret_cast<Real *>(sp_smem);   // N x (W + 1)
+    const int axis = axis0 + blockIdx.y;
+    const Real *__restrict__ u = u0 + blockIdx.y * stride;
     const int W = sp_lines<Real>(N);
     const int ld = W + 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    double acc[MPW][PMAX];
+    const int all = (nr + kSpPerWarp - 1) / kSpPerWarp, ngroups = min(kSpGroups, all);
+    const int group = (int)blockIdx.z * kSpGroups + warp % ngroups;
+    // a lane's line, and the share of the positions that its part of the warp and its warp take
+    const int per = 32 / W, line = lane % W, sub = lane / W;
+    const int first = (warp / ngroups) * per + sub, pstep = (nwarps / ngroups) * per;
+    double acc[kSpPerWarp][PMAX];
+    int rr[kSpPerWarp];
 #pragma unroll
-    for (int a = 0; a < MPW; ++a)
+    for (int a = 0; a < kSpPerWarp; ++a) {
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) acc[a][p] = 0.0;
-    int rr[MPW];
-#pragma unroll
-    for (int a = 0; a < MPW; ++a) {
-        const int m = warp + a * nwarps;
-        rr[a] = m < nr ? rs[m] % N : -1;
+        const int m = group * kSpPerWarp + a;
+        rr[a] = m < nr ? rs[m] : 0;   // a separation of zero adds zeros
     }
     // axis 0: groups of W consecutive x-rows (row = y + n1 z); axes 1, 2: groups of W
     // consecutive x at fixed z (axis 1) or fixed y (axis 2)
     const int xgroups = (n0 + W - 1) / W;
     const int64_t nrows = (int64_t)n1 * n2;
-    const int64_t ngroups = axis == 0 ? (nrows + W - 1) / W : (int64_t)xgroups * (axis == 1 ? n2 : n1);
-    for (int64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
+    const int64_t ntiles = axis == 0 ? (nrows + W - 1) / W : (int64_t)xgroups * (axis == 1 ? n2 : n1);
+    for (int64_t g = blockIdx.x; g < ntiles; g += gridDim.x) {
         __syncthreads();
-        int nl;   // lines of this group
+        int nl;   // lines of this tile
         if (axis == 0) {
             const int64_t row0 = g * W;
             nl = (int)min((int64_t)W, nrows - row0);
-            for (int e = threadIdx.x; e < N * nl; e += blockDim.x) {
-                const int x = e % N, l = e / N;
-                tile[x * ld + l] = u[(size_t)(row0 + l) * n0 + x];
-            }
+            for (int l = warp; l < nl; l += nwarps)
+                for (int x = lane; x < N; x += 32) tile[x * ld + l] = u[(size_t)(row0 + l) * n0 + x] * sc;
         } else {
             const int xg = (int)(g % xgroups), o = (int)(g / xgroups);
             const int x0 = xg * W;
             nl = min(W, n0 - x0);
-            for (int e = threadIdx.x; e < N * W; e += blockDim.x) {
-                const int l = e % W, pos = e / W;
-                if (l >= nl) continue;
-                size_t gi;
-                if (axis == 1) gi = (size_t)(x0 + l) + (size_t)n0 * ((size_t)pos + (size_t)n1 * o);
-                else gi = (size_t)(x0 + l) + (size_t)n0 * ((size_t)o + (size_t)n1 * pos);
-                tile[pos * ld + l] = u[gi];
-            }
+            const size_t base = axis == 1 ? (size_t)n0 * ((size_t)n1 * o) : (size_t)n0 * o;
+            const size_t ps = axis == 1 ? (size_t)n0 : (size_t)n0 * n1;
+            if (line < nl && sub < per)
+                for (int pos = warp * per + sub; pos < N; pos += nwarps * per)
+                    tile[pos * ld + line] = u[base + ps * pos + x0 + line] * sc;
         }
         __syncthreads();
-        if (lane < nl) {
+        if (line < nl && sub < per) {
+            for (int pos = first; pos < N; pos += pstep) {
+                const double c = (double)tile[pos * ld + line];
 #pragma unroll
-            for (int a = 0; a < MPW; ++a) {
-                const int r = rr[a];
-                if (r < 0) continue;
-                for (int pos = 0; pos < N; ++pos) {
-                    int q = pos + r;
+                for (int a = 0; a < kSpPerWarp; ++a) {
+                    int q = pos + rr[a];
                     if (q >= N) q -= N;
-                    const double du = ((double)tile[q * ld + lane] - (double)tile[pos * ld + lane]) * s;
-                    double pw = du;
-#pragma unroll
-                    for (int p = 0; p < PMAX; ++p) {
-                        acc[a][p] += pw;
-                        pw *= du;
-                    }
+                    sp_accumulate<PMAX>((double)tile[q * ld + line] - c, acc[a]);
                 }
             }
         }
     }
 #pragma unroll
-    for (int a = 0; a < MPW; ++a) {
-        const int m = warp + a * nwarps;
-        if (m >= nr) continue;
+    for (int a = 0; a < kSpPerWarp; ++a) {
+        const int m = group * kSpPerWarp + a;
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) {
             const double v = warp_sum(acc[a][p]);
-            if (lane == 0) atomicAdd(Sp + p * nr + m, v);
+            if (lane == 0 && m < nr) atomicAdd(Sp + p * nr + m, v);
         }
     }
 }
@@ -214,14 +295,11 @@ int stats_minmax(Ctx *c, int which)
     char *mm = (char *)c->scratch[19].p + 16;
     const int km = kt_begin(c, KT_STATS);
     mm_init2<<<1, 32, 0, c->stream>>>(mm, 6, wide ? 1 : 0);
-    for (int d = 0; d < 3; ++d) {
-        if (wide)
-            minmax_kernel<double><<<grid_for(c, n3), 256, 0, c->stream>>>((const double *)f + d * n3, n3, mm + 16 * d);
-        else
-            minmax_kernel<float><<<grid_for(c, n3), 256, 0, c->stream>>>((const float *)f + d * n3, n3, mm + 8 * d);
-    }
+    const dim3 g(grid_for(c, n3 / (wide ? 2 : 4), 4), 3);
+    if (wide) minmax_kernel<double><<<g, 256, 0, c->stream>>>((const double *)f, n3, mm);
+    else minmax_kernel<float><<<g, 256, 0, c->stream>>>((const float *)f, n3, mm);
     kt_end(c, km);
-    c->launches += 4;
+    c->launches += 2;
     FWT_CUDA(cudaGetLastError());
     unsigned long long h[6];
     FWT_CUDA(cudaMemcpyAsync(h, mm, wide ? 48 : 24, cudaMemcpyDeviceToHost, c->stream));
@@ -300,7 +378,10 @@ int stats_pdf(Ctx *c, int which, int comp, int nbins, float *val, float *pdf, ui
     FWT_CUDA(cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long) * nbins, c->stream));
     const size_t n3 = field_elems(c);
     const void *f = is_u ? c->b_u.p : c->b_w.p;
-    const size_t shb = sizeof(float) * 2 * nbins + sizeof(uint32_t) * nbins;
+    // copies of the counts: as many as fit 40 KB beside the edges, up to one per lane
+    int copies = 1;
+    while (copies < 32 && sizeof(float) * nbins * (2 + 2 * (size_t)copies) <= 40960) copies *= 2;
+    const size_t shb = sizeof(float) * 2 * nbins + sizeof(uint32_t) * nbins * (size_t)copies;
     // 8192 bins take 96 KB of shared memory, above the default 48 KB: the limit is raised to
     // the device's opt-in maximum, the same value for every context (the attribute belongs to
     // the kernel, for the whole process)
@@ -312,16 +393,16 @@ int stats_pdf(Ctx *c, int which, int comp, int nbins, float *val, float *pdf, ui
     else
         FWT_CUDA(cudaFuncSetAttribute(pdf_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     const int km = kt_begin(c, KT_STATS);
-    for (int d = 0; d < 3; ++d) {
-        if (comp >= 0 && d != comp) continue;
-        if (c->p.precision == 64)
-            pdf_kernel<double><<<grid_for(c, n3, 4), 256, shb, c->stream>>>((const double *)f + d * n3, n3, s, d_lo,
-                                                                            d_hi, nbins, d_cnt);
-        else
-            pdf_kernel<float><<<grid_for(c, n3, 4), 256, shb, c->stream>>>((const float *)f + d * n3, n3, s, d_lo,
-                                                                           d_hi, nbins, d_cnt);
-        c->launches += 1;
-    }
+    // the components lie one after the other: one launch takes one of them or all three
+    const size_t o = comp < 0 ? 0 : (size_t)comp * n3, nv = comp < 0 ? 3 * n3 : n3;
+    const float ibsz = bsz > 0.0f ? 1.0f / bsz : 0.0f;
+    if (c->p.precision == 64)
+        pdf_kernel<double><<<grid_for(c, nv / 2, 4), 256, shb, c->stream>>>((const double *)f + o, nv, s, vmin, ibsz, d_lo,
+                                                                            d_hi, nbins, copies, d_cnt);
+    else
+        pdf_kernel<float><<<grid_for(c, nv / 4, 4), 256, shb, c->stream>>>((const float *)f + o, nv, s, vmin, ibsz, d_lo,
+                                                                           d_hi, nbins, copies, d_cnt);
+    c->launches += 1;
     kt_end(c, km);
     FWT_CUDA(cudaGetLastError());
     std::vector<unsigned long long> hc(nbins);
@@ -342,6 +423,74 @@ int stats_pdf(Ctx *c, int which, int comp, int nbins, float *val, float *pdf, ui
     return 0;
 }
 
+// Sums of du^p, p = 1..pmax, on a box (n0 x n1 x n2) of `axes` consecutive axes from axis0 (one
+// component each, `stride` elements apart): sums[(p - 1) * nr + m] = sum (du s)^p at separation
+// r[m].  Separations equal modulo N are summed once.
+static int sp_sums(Ctx *c, const void *u, size_t stride, int n0, int n1, int n2, int axis0, int axes, double s, int pmax,
+                   const int *r, int nr, double *sums)
+{
+    const int N = c->p.N;
+    const bool f64 = c->p.precision == 64;
+    const int W = f64 ? sp_lines<double>(N) : sp_lines<float>(N);
+    const size_t shb = (f64 ? sizeof(double) : sizeof(float)) * (size_t)N * (W + 1);
+    // The dynamic shared-memory limit is a property of the kernel for the whole process: every
+    // context sets the same value, the device's opt-in maximum, so that contexts of different N
+    // on concurrent host threads never lower it under another's launch.
+    int optin = 0;
+    FWT_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->dev));
+    if (shb > (size_t)optin) return fail(FWT_E_RANGE, "Sp: N too large for one block's shared memory");
+    std::vector<int> uniq, at(nr);
+    for (int m = 0; m < nr; ++m) {
+        const int q = r[m] % N;
+        size_t i = 0;
+        while (i < uniq.size() && uniq[i] != q) ++i;
+        if (i == uniq.size()) uniq.push_back(q);
+        at[m] = (int)i;
+    }
+    const int P = pmax <= 4 ? 4 : (pmax <= 6 ? 6 : 10), nu = (int)uniq.size();
+    std::vector<double> h((size_t)P * nu);
+    // the power of two nearest 1 / s scales the staged lines exactly; the rest is applied below
+    int e = 0;
+    std::frexp(s, &e);
+    const double sc = std::isfinite(s) && s > 0 && e > -100 && e < 100 ? std::ldexp(1.0, e) : 1.0;
+    FWT_TRY(buf_reserve(c, c->scratch[9], sizeof(int) * 64 + sizeof(double) * 10 * 64 + 64));
+    int *d_r = (int *)c->scratch[9].p;
+    double *d_sp = (double *)((char *)c->scratch[9].p + 256);
+    FWT_CUDA(cudaMemcpyAsync(d_r, uniq.data(), sizeof(int) * nu, cudaMemcpyHostToDevice, c->stream));
+    FWT_CUDA(cudaMemsetAsync(d_sp, 0, sizeof(double) * P * nu, c->stream));
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
+    const int64_t tiles = (int64_t)n0 * n1 * n2 / N / W + 1;
+    const int all = (nu + kSpPerWarp - 1) / kSpPerWarp, ngroups = std::min(kSpGroups, all);
+    const unsigned threads = 32u * (unsigned)(ngroups <= 6 ? 2 * ngroups : ngroups);
+    const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)sms * 2)), (unsigned)axes,
+                    (unsigned)((all + kSpGroups - 1) / kSpGroups));
+    const int km = kt_begin(c, KT_STATS);
+#define FWT_SP(REAL, PM)                                                                                           \
+do {                                                                                                           \
+    auto k = sp_kernel<REAL, PM>;                                                                              \
+    FWT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));                    \
+    k<<<grid, threads, shb, c->stream>>>((const REAL *)u, stride, N, n0, n1, n2, axis0, (REAL)sc, d_r, nu, d_sp); \
+} while (0)
+    if (f64) {
+        if (P == 4) FWT_SP(double, 4); else if (P == 6) FWT_SP(double, 6); else FWT_SP(double, 10);
+    } else {
+        if (P == 4) FWT_SP(float, 4); else if (P == 6) FWT_SP(float, 6); else FWT_SP(float, 10);
+    }
+#undef FWT_SP
+    kt_end(c, km);
+    c->launches += 1;
+    FWT_CUDA(cudaGetLastError());
+    FWT_CUDA(cudaMemcpyAsync(h.data(), d_sp, sizeof(double) * P * nu, cudaMemcpyDeviceToHost, c->stream));
+    FWT_CUDA(cudaStreamSynchronize(c->stream));
+    double f = 1.0;
+    for (int p = 0; p < pmax; ++p) {
+        f *= s / sc;
+        for (int m = 0; m < nr; ++m) sums[p * nr + m] = h[(size_t)p * nu + at[m]] * f;
+    }
+    return 0;
+}
+
 int stats_sp(Ctx *c, int pmax, const int *r, int nr, double *Sp)
 {
     if (c->slab_nz) return fail(FWT_E_STATE, "S_p: not available on a z-slab context");
@@ -349,54 +498,11 @@ int stats_sp(Ctx *c, int pmax, const int *r, int nr, double *Sp)
     if (pmax < 1 || pmax > 10) return fail(FWT_E_ARG, "Sp: pmax must be 1..10");
     if (nr < 1 || nr > 64) return fail(FWT_E_ARG, "Sp: nr must be 1..64");
     const int N = c->p.N;
-    const bool f64 = c->p.precision == 64;
-    const int W = f64 ? sp_lines<double>(N) : sp_lines<float>(N);
     for (int m = 0; m < nr; ++m)
         if (r[m] < 0) return fail(FWT_E_ARG, "Sp: negative separation");
-    FWT_TRY(buf_reserve(c, c->scratch[9], sizeof(int) * 64 + sizeof(double) * 10 * 64 + 64));
-    int *d_r = (int *)c->scratch[9].p;
-    double *d_sp = (double *)((char *)c->scratch[9].p + 256);
-    FWT_CUDA(cudaMemcpyAsync(d_r, r, sizeof(int) * nr, cudaMemcpyHostToDevice, c->stream));
-    FWT_CUDA(cudaMemsetAsync(d_sp, 0, sizeof(double) * 10 * nr, c->stream));
-    const size_t n3 = field_elems(c);
-    const double s = 1.0 / c->up;
-    const size_t shb = (f64 ? sizeof(double) : sizeof(float)) * (size_t)N * (W + 1);
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
-    const int64_t groups = ((int64_t)N * N + W - 1) / W;
-    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(groups, (int64_t)sms * 4));
-    const int mpw = (nr + 7) / 8;
-    // The dynamic shared-memory limit is a property of the kernel for the whole process: every
-    // context sets the same value, the device's opt-in maximum, so that contexts of different N
-    // on concurrent host threads never lower it under another's launch.
-    int optin = 0;
-    FWT_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->dev));
-    if (shb > (size_t)optin) return fail(FWT_E_RANGE, "Sp: N too large for one block's shared memory");
-    const int km = kt_begin(c, KT_STATS);
-#define FWT_SP(REAL, MPW)                                                                                        \
-    do {                                                                                                         \
-        auto k = sp_kernel<REAL, 10, MPW>;                                                                       \
-        FWT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));                  \
-        for (int ax = 0; ax < 3; ++ax)                                                                           \
-            k<<<blocks, 256, shb, c->stream>>>((const REAL *)c->b_u.p + ax * n3, N, N, N, N, ax, s, d_r, nr, d_sp); \
-    } while (0)
-    if (c->p.precision == 64) {
-        if (mpw <= 1) FWT_SP(double, 1); else if (mpw <= 2) FWT_SP(double, 2); else if (mpw <= 4) FWT_SP(double, 4);
-        else FWT_SP(double, 8);
-    } else {
-        if (mpw <= 1) FWT_SP(float, 1); else if (mpw <= 2) FWT_SP(float, 2); else if (mpw <= 4) FWT_SP(float, 4);
-        else FWT_SP(float, 8);
-    }
-#undef FWT_SP
-    kt_end(c, km);
-    c->launches += 3;
-    FWT_CUDA(cudaGetLastError());
-    std::vector<double> h(10 * nr);
-    FWT_CUDA(cudaMemcpyAsync(h.data(), d_sp, sizeof(double) * 10 * nr, cudaMemcpyDeviceToHost, c->stream));
-    FWT_CUDA(cudaStreamSynchronize(c->stream));
+    FWT_TRY(sp_sums(c, c->b_u.p, field_elems(c), N, N, N, 0, 3, 1.0 / c->up, pmax, r, nr, Sp));
     const double inv = 1.0 / ((double)N * N * N * 3.0);
-    for (int p = 0; p < pmax; ++p)
-        for (int m = 0; m < nr; ++m) Sp[p * nr + m] = h[p * nr + m] * inv;
+    for (int i = 0; i < pmax * nr; ++i) Sp[i] *= inv;
     return 0;
 }
 
@@ -467,43 +573,7 @@ int stats_sp_block(Ctx *c, const void *u, int n0, int n1, int n2, int axis, doub
     if (nr < 1 || nr > 64) return fail(FWT_E_ARG, "sp_block: nr must be 1..64");
     for (int m = 0; m < nr; ++m)
         if (r[m] < 0) return fail(FWT_E_ARG, "sp_block: negative separation");
-    const bool f64 = c->p.precision == 64;
-    const int W = f64 ? sp_lines<double>(N) : sp_lines<float>(N);
-    FWT_TRY(buf_reserve(c, c->scratch[9], sizeof(int) * 64 + sizeof(double) * 10 * 64 + 64));
-    int *d_r = (int *)c->scratch[9].p;
-    double *d_sp = (double *)((char *)c->scratch[9].p + 256);
-    FWT_CUDA(cudaMemcpyAsync(d_r, r, sizeof(int) * nr, cudaMemcpyHostToDevice, c->stream));
-    FWT_CUDA(cudaMemsetAsync(d_sp, 0, sizeof(double) * 10 * nr, c->stream));
-    const size_t shb = (f64 ? sizeof(double) : sizeof(float)) * (size_t)N * (W + 1);
-    int optin = 0;
-    FWT_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->dev));
-    if (shb > (size_t)optin) return fail(FWT_E_RANGE, "sp_block: N too large for one block's shared memory");
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
-    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)n0 * n1 * n2 / N / W + 1,
-                                                                             (int64_t)sms * 4));
-    const int mpw = (nr + 7) / 8;
-    const int km = kt_begin(c, KT_STATS);
-#define FWT_SPB(REAL, MPW)                                                                                       \
-    do {                                                                                                         \
-        auto k = sp_kernel<REAL, 10, MPW>;                                                                       \
-        FWT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));                  \
-        k<<<blocks, 256, shb, c->stream>>>((const REAL *)u, N, n0, n1, n2, axis, s, d_r, nr, d_sp);              \
-    } while (0)
-    if (f64) {
-        if (mpw <= 1) FWT_SPB(double, 1); else if (mpw <= 2) FWT_SPB(double, 2); else if (mpw <= 4) FWT_SPB(double, 4);
-        else FWT_SPB(double, 8);
-    } else {
-        if (mpw <= 1) FWT_SPB(float, 1); else if (mpw <= 2) FWT_SPB(float, 2); else if (mpw <= 4) FWT_SPB(float, 4);
-        else FWT_SPB(float, 8);
-    }
-#undef FWT_SPB
-    kt_end(c, km);
-    c->launches += 1;
-    FWT_CUDA(cudaGetLastError());
-    FWT_CUDA(cudaMemcpyAsync(sums, d_sp, sizeof(double) * 10 * nr, cudaMemcpyDeviceToHost, c->stream));
-    FWT_CUDA(cudaStreamSynchronize(c->stream));
-    return 0;
+    return sp_sums(c, u, 0, n0, n1, n2, axis, 1, s, 10, r, nr, sums);
 }
 
 }  // namespace fwt
