@@ -1,9 +1,9 @@
 // k_centerline.cu -- centerline set-up on the device, all FP64 (one B200 runs FP64 at half
 // the FP32 rate, and the integer sub-segment counts must follow the reference):
 //   line_prep_kernel   periodic arc length cze, Len_Disc, c', c''       tube.f90:392-515
-//   section_coe_kernel quintic coefficients                              subroutine.f90:440-488
-//   section_kernel     turning-angle sum, one warp per section           tube.f90:625-657
-//   section_ntf_kernel ntf/dtf, FP64 recompute list near a step of ceil  tube.f90:655-657
+//   section_coe_kernel quintic coefficients, sub-segment count           subroutine.f90:440-488
+//   section_fine_kernel, section_kernel, section_fp64_kernel: the counts  tube.f90:625-657
+//                      that a coarser sum leaves open
 //   sample_kernel      sample points ci with the endpoint copy          tube.f90:706-723
 //   chord_kernel       chords dci, |dci|, unit chords tci               tube.f90:740-751
 //   subseg_kernel      sub-segment records (unwrap, Rtube, box)          tube.f90:766-798
@@ -121,10 +121,10 @@ __global__ void line_prep_kernel(const LineParam *__restrict__ lp, int nlines, c
 
 
 // ------------------------------------------------------------------ a3/a5: sections
-// |c' x c''| / |c'|^2 at z of the quintic whose derivative coefficients are d1 ([coord][5]:
-// a1, 2 a2, 3 a3, 4 a4, 5 a5) and d2 ([coord][4]: 2 a2, 6 a3, 12 a4, 20 a5), FP32
-// (tube.f90:633-647), added to th
-__device__ __forceinline__ void turning_integrand(const float (&d1)[3][5], const float (&d2)[3][4], float z, float &th)
+// |c' x c''| / |c'|^2 (returned) and |c'|^2 (q) at z of the quintic whose derivative coefficients
+// are d1 ([coord][5]: a1, 2 a2, 3 a3, 4 a4, 5 a5) and d2 ([coord][4]: 2 a2, 6 a3, 12 a4, 20 a5), FP32
+// (tube.f90:633-647)
+__device__ __forceinline__ float turning_integrand(const float (&d1)[3][5], const float (&d2)[3][4], float z, float &q)
 {
     float dc[3], dd[3];
 #pragma unroll
@@ -135,29 +135,124 @@ __device__ __forceinline__ void turning_integrand(const float (&d1)[3][5], const
     const float x0 = dc[1] * dd[2] - dc[2] * dd[1];
     const float x1 = dc[2] * dd[0] - dc[0] * dd[2];
     const float x2 = dc[0] * dd[1] - dc[1] * dd[0];
-    const float ndc2 = dc[0] * dc[0] + dc[1] * dc[1] + dc[2] * dc[2];
+    q = dc[0] * dc[0] + dc[1] * dc[1] + dc[2] * dc[2];
     // hardware square root and reciprocal (a few ulp): the sum only has to land within 1e-4 of
     // the reference's, and sections closer than that to a step of ceil() are redone in FP64
     float nx, rn;
     asm("sqrt.approx.f32 %0, %1;" : "=f"(nx) : "f"(x0 * x0 + x1 * x1 + x2 * x2));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rn) : "f"(ndc2));
-    th = fmaf(nx, rn, th);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rn) : "f"(q));
+    return nx * rn;
 }
 
-// Sections in three passes (n_sec + 1 slots per line; slot n_sec is the periodic copy): the
-// quintic coefficients and the sample step, one thread per slot (section_coe_kernel); the
-// turning-angle sum, one warp per slot (section_kernel); ntf and dtf, one thread per slot
-// (section_ntf_kernel).  The FP64 arithmetic of the first and last pass runs on every lane
-// instead of three lanes of the summing warp.
+// The reference counts a section's sub-segments from the sum of the turning angle over ntf_pre + 1
+// samples (1001): ntf = ceil(ntf_times theta / 2 pi) + 1, an integer, so theta is needed only well
+// enough to tell which step of ceil it falls on.  The sections (n_sec + 1 slots per line; slot
+// n_sec is the periodic copy) are decided by ever finer quadratures, each with a bound on its
+// error; a section whose bound straddles a step goes to the next one's list:
+//   1. section_coe_kernel   one thread per section: coefficients (FP64), 64 intervals
+//   2. section_fine_kernel  one thread per listed section: 256 intervals
+//   3. section_kernel       one warp per listed section: the reference's own sum in FP32
+//   4. section_fp64_kernel  one warp per listed section: the reference's sum in FP64
+// Bound by FP32 issue: step 3 takes 1500 warp instructions a section, step 1 about 110.  With every
+// section in step 3 (and 4) the 38 M sections of a six-level field (H = 0.7) took 68 ms; the four
+// together take 9.7 ms (5.6, 2.5, 1.0, 0.6).
+//
+// The bound.  With h the sample spacing, the trapezoidal sum of a smooth integrand f is off by
+// about h / 12 sum |second differences of f|, and so is that of a kink (|c' x c''| passing near
+// zero) or of any feature wider than h; Simpson's rule, which is used, is rarely off by as much.
+// What the samples cannot show is a peak of 1 / |c'|^2 between two of them: a zero of the positive
+// polynomial |c'|^2 at a distance b from the section in the complex plane gives |c'|^2 a second
+// difference of 2 h^2 / (d^2 + b^2) of itself at a sample d <= h / 2 away, so where no second
+// difference exceeds a tenth of |c'|^2 every b is above 4 h and the peaks are resolved; where one
+// does, the section counts as undecided.  Twice the bound is allowed for: over 1.1 M sections of
+// fractional bridges with H from 0.3 to 0.8 the sum's distance from the reference's stayed below
+// 0.47 of it.  The reference's sum itself is a trapezoidal sum with ntf_pre intervals plus half the
+// end values: ntf_pre >= 512 keeps its own distance from the integral far below the bound; smaller
+// values go to step 3 at once.
+constexpr int kQuadMinPre = 512;
 
-// get_spline_5th_coe (subroutine.f90:440-461) for the three coordinates of slot s, and the FP32
-// sample step dtf_pre * Len of the turning-angle sum.
-__global__ void section_coe_kernel(const LineParam *__restrict__ lp, const int *__restrict__ slot_line, int64_t nslots,
-                                   const double *__restrict__ X, const double *__restrict__ Y,
-                                   const double *__restrict__ Z, const double *__restrict__ cze,
-                                   const double *__restrict__ ck, const double *__restrict__ ckk,
-                                   const double *__restrict__ Len, int64_t node_base, int ntf_pre,
-                                   double *__restrict__ coe_out, float *__restrict__ zstep_out)
+struct SectionSum {
+    float tsum, err;   // sum over the reference's samples (without the step), bound of its error
+    bool resolved;
+};
+
+template <int Intervals>
+__device__ __forceinline__ SectionSum section_quadrature(const float (&d1)[3][5], const float (&d2)[3][4], float zr,
+                                                         int ntf_pre)
+{
+    const float h = 1.0f / Intervals, dz = zr * h;
+    float q0, q1, q2;
+    float f0 = turning_integrand(d1, d2, 0.0f, q0), f1 = turning_integrand(d1, d2, dz, q1);
+    const float fa = f0, qa = q0;
+    float odd = f1, even = 0.0f, dd = 0.0f;   // interior sums, sum of |second differences|
+    float qx = 0.0f;                          // the first end's second difference
+    bool rough = false;
+#pragma unroll 2
+    for (int i = 2; i <= Intervals; ++i) {
+        const float f2 = turning_integrand(d1, d2, dz * (float)i, q2);
+        dd += fabsf((f0 - f1) + (f2 - f1));
+        const float e = (q0 - q1) + (q2 - q1);
+        rough = rough || !(e <= 0.1f * q1);
+        if (i == 2) qx = e;
+        if (i == Intervals) rough = rough || !(e <= 0.1f * q2);
+        if (i < Intervals) {
+            if (i & 1) odd += f2;
+            else even += f2;
+        }
+        f0 = f1;
+        f1 = f2;
+        q0 = q1;
+        q1 = q2;
+    }
+    rough = rough || !(qx <= 0.1f * qa);
+    SectionSum s;
+    // n_pre times Simpson's integral over the unit interval, plus half the end values
+    s.tsum = fmaf((fa + f1 + 4.0f * odd + 2.0f * even) * (h / 3.0f), (float)ntf_pre, 0.5f * (fa + f1));
+    s.err = (2.0f / 12.0f) * h * dd * (float)ntf_pre;
+    s.resolved = !rough;
+    return s;
+}
+
+// Decide a slot from its sum, or leave it to the next list: 0 decided, 1 the quadrature's bound
+// straddles a step, 2 only the FP32 rounding (1e-4) does.
+__device__ __forceinline__ int section_decide(const SectionSum &q, double dtfp, double L, int ntf_times, int &ntf)
+{
+    const double k = dtfp * L * ntf_times / dev_pi2();
+    const double x = (double)q.tsum * k, rounding = 1e-4 * (x + 1.0), e = (double)q.err * k;
+    if (!q.resolved || !(x == x) || !(e == e)) return 1;
+    const double m = e + rounding;
+    if (floor(x + m) == floor(x - m)) {
+        ntf = (int)ceil(x) + 1;
+        return 0;
+    }
+    return e <= 0.1 * rounding ? 2 : 1;
+}
+
+// The lists of undecided slots: three of them, each its counter and its slots.
+struct SectionLists {
+    unsigned *count;        // [0] fine, [1] full sum, [2] FP64
+    unsigned *fine, *full, *fp64;
+};
+
+__device__ __forceinline__ void list_push(unsigned *count, unsigned *list, bool put, unsigned slot)
+{
+    const unsigned act = __activemask(), bal = __ballot_sync(act, put);
+    if (!put) return;
+    const int lane = threadIdx.x & 31, leader = __ffs(bal) - 1;
+    unsigned base = 0;
+    if (lane == leader) base = atomicAdd(count, (unsigned)__popc(bal));
+    base = __shfl_sync(bal, base, leader);
+    list[base + __popc(bal & ((1u << lane) - 1u))] = slot;
+}
+
+// get_spline_5th_coe (subroutine.f90:440-461) for the three coordinates of slot s, the FP32 sample
+// step dtf_pre * Len of the turning-angle sum, and the slot's ntf and dtf where 64 intervals decide.
+__global__ void __launch_bounds__(256) section_coe_kernel(
+    const LineParam *__restrict__ lp, const int *__restrict__ slot_line, int64_t nslots, const double *__restrict__ X,
+    const double *__restrict__ Y, const double *__restrict__ Z, const double *__restrict__ cze,
+    const double *__restrict__ ck, const double *__restrict__ ckk, const double *__restrict__ Len, int64_t node_base,
+    int ntf_times, int ntf_pre, double *__restrict__ coe_out, float *__restrict__ zstep_out, int *__restrict__ ntf_out,
+    double *__restrict__ dtf_out, const SectionLists lists)
 {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nslots) return;
@@ -175,7 +270,8 @@ __global__ void section_coe_kernel(const LineParam *__restrict__ lp, const int *
     // spline argument is cze_pl*Len (tube.f90:598)
     const double zr = zr_ * L - zl * L;
     const double z2 = zr * zr, z3 = z2 * zr, z4 = z3 * zr, z5 = z4 * zr;
-#pragma unroll 1
+    float d1[3][5], d2[3][4];
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
         const double *cd = (d == 0 ? X : (d == 1 ? Y : Z)) + P.node_off;
         const double xl = cd[il], xr = cd[ir];
@@ -184,97 +280,143 @@ __global__ void section_coe_kernel(const LineParam *__restrict__ lp, const int *
         double xpl = xl, xpr = xr;
         if (xl - xr > dev_pi()) xpr = xr + dev_pi2();
         else if (xl - xr < -dev_pi()) xpl = xl + dev_pi2();
-        double *a6 = coe_out + 18 * s + 6 * d;
+        double a6[6];
         a6[0] = xl;
         a6[1] = vl;
         a6[2] = al / 2.0;
         a6[3] = (20.0 * (xpr - xpl) - (12.0 * vl + 8.0 * vr) * zr - (3.0 * al - ar) * z2) / (2.0 * z3);
         a6[4] = (-30.0 * (xpr - xpl) + (16.0 * vl + 14.0 * vr) * zr + (3.0 * al - 2.0 * ar) * z2) / (2.0 * z4);
         a6[5] = (12.0 * (xpr - xpl) - 6.0 * (vl + vr) * zr - (al - ar) * z2) / (2.0 * z5);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) coe_out[18 * s + 6 * d + m] = a6[m];
+#pragma unroll
+        for (int m = 1; m <= 5; ++m) d1[d][m - 1] = (float)m * (float)a6[m];
+#pragma unroll
+        for (int m = 2; m <= 5; ++m) d2[d][m - 2] = (float)(m * (m - 1)) * (float)a6[m];
     }
     const double dtfp = (zr_ - zl) / (1.0 * ntf_pre);
     zstep_out[s] = (float)(dtfp * L);
-}
-
-// The turning-angle sum of slot `warp` (tube.f90:625-657): sum |c' x c''| / |c'|^2 over
-// ntf_pre + 1 samples, the integrand in FP32 from the FP32 coefficients, the sum in FP64
-// (without the factor dtf_pre * Len, applied by section_ntf_kernel).
-__global__ void section_kernel(int64_t nslots, int ntf_pre, const double *__restrict__ coe,
-                               const float *__restrict__ zstep_in, double *__restrict__ tsum_out)
-{
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= nslots) return;
-    // lane m < 18 loads coefficient m; every lane takes the FP32 derivative coefficients by
-    // shuffles, scaled once (1, 2, 3, 4, 5 for c' and 2, 6, 12, 20 for c'')
-    const float mine = lane < 18 ? (float)coe[18 * warp + lane] : 0.0f;
-    float d1[3][5], d2[3][4];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-#pragma unroll
-        for (int m = 1; m <= 5; ++m) d1[d][m - 1] = (float)m * __shfl_sync(0xffffffffu, mine, 6 * d + m);
-#pragma unroll
-        for (int m = 2; m <= 5; ++m) d2[d][m - 2] = (float)(m * (m - 1)) * __shfl_sync(0xffffffffu, mine, 6 * d + m);
-    }
-    const float zstep = zstep_in[warp], z64 = 64.0f * zstep;
-    float th0 = 0.0f, th1 = 0.0f;
-    int tj = lane;
-    float za = zstep * (float)lane, zb = zstep * (float)(lane + 32);
-    for (; tj + 32 <= ntf_pre; tj += 64) {   // two independent samples per step
-        turning_integrand(d1, d2, za, th0);
-        turning_integrand(d1, d2, zb, th1);
-        za += z64;
-        zb += z64;
-    }
-    if (tj <= ntf_pre) turning_integrand(d1, d2, za, th0);
-    const double sum = warp_sum((double)th0 + (double)th1);
-    if (lane == 0) tsum_out[warp] = sum;
-}
-
-// ntf = ceil(ntf_times theta / 2 pi) + 1 and dtf of slot s, theta = sum * dtf_pre * Len.  The
-// integrand was evaluated in FP32; a result that falls near a step of ceil is marked (ntf = 0)
-// and recomputed in FP64 by section_fp64_kernel.
-__global__ void section_ntf_kernel(const LineParam *__restrict__ lp, const int *__restrict__ slot_line, int64_t nslots,
-                                   const double *__restrict__ cze, const double *__restrict__ Len, int64_t node_base,
-                                   int ntf_times, int ntf_pre, const double *__restrict__ tsum,
-                                   int *__restrict__ ntf_out, double *__restrict__ dtf_out,
-                                   unsigned *__restrict__ near)   // near[0]: count, near[4 + i]: marked slots
-{
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nslots) return;
-    const int l = slot_line[s];
-    const LineParam P = lp[l];
-    const int t = (int)(s - P.slot_off);
-    const int np = P.n_sec;
-    const double L = Len[l];
-    const double *cz_line = cze + (P.node_off - node_base);
-    const double zl = cze_pl_at(cz_line, np, t), zr_ = cze_pl_at(cz_line, np, t + 1);
-    const double dtfp = (zr_ - zl) / (1.0 * ntf_pre);
-    const double th32 = tsum[s] * dtfp * L;
-    const double xr = ntf_times * th32 / dev_pi2();
-    const double fr = xr - floor(xr);
-    const bool near_step = fmin(fr, 1.0 - fr) < 1e-4 * (xr + 1.0) || !(xr == xr);
-    const int ntf = near_step ? 0 : (int)ceil(xr) + 1;
-    if (near_step) near[4 + atomicAdd(near, 1u)] = (unsigned)s;
+    int left = 1, ntf = 0;
+    if (ntf_pre >= kQuadMinPre)
+        left = section_decide(section_quadrature<64>(d1, d2, (float)zr, ntf_pre), dtfp, L, ntf_times, ntf);
     ntf_out[s] = ntf;
-    dtf_out[s] = near_step ? 0.0 : (zr_ - zl) / (1.0 * ntf);
+    dtf_out[s] = left == 0 ? (zr_ - zl) / (1.0 * ntf) : 0.0;
+    const bool fine = left == 1 && ntf_pre >= kQuadMinPre;
+    list_push(lists.count, lists.fine, fine, (unsigned)s);
+    list_push(lists.count + 1, lists.full, left == 1 && !fine, (unsigned)s);
+    list_push(lists.count + 2, lists.fp64, left == 2, (unsigned)s);
 }
 
-// FP64 turning angle of the sections section_kernel marked (ntf = 0), taken from its list of
-// them (a few per thousand): a fixed grid of warps strides over the list, one section per warp
-// at a time, with the reference's integrand (tube.f90:625-657) in FP64 from the stored
+// The sections of the first list with 256 intervals.
+__global__ void __launch_bounds__(128) section_fine_kernel(const LineParam *__restrict__ lp,
+                                                           const int *__restrict__ slot_line,
+                                                           const double *__restrict__ cze, const double *__restrict__ Len,
+                                                           int64_t node_base, int ntf_times, int ntf_pre,
+                                                           const double *__restrict__ coe, int *__restrict__ ntf_out,
+                                                           double *__restrict__ dtf_out, const SectionLists lists)
+{
+    const unsigned n = lists.count[0];
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const unsigned s = lists.fine[i];
+        const int l = slot_line[s];
+        const LineParam P = lp[l];
+        const int t = (int)(s - P.slot_off), np = P.n_sec;
+        const double L = Len[l];
+        const double *cz_line = cze + (P.node_off - node_base);
+        const double zl = cze_pl_at(cz_line, np, t), zr_ = cze_pl_at(cz_line, np, t + 1);
+        float d1[3][5], d2[3][4];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+#pragma unroll
+            for (int m = 1; m <= 5; ++m) d1[d][m - 1] = (float)m * (float)coe[18 * (size_t)s + 6 * d + m];
+#pragma unroll
+            for (int m = 2; m <= 5; ++m) d2[d][m - 2] = (float)(m * (m - 1)) * (float)coe[18 * (size_t)s + 6 * d + m];
+        }
+        const double dtfp = (zr_ - zl) / (1.0 * ntf_pre);
+        int ntf = 0;
+        const int left = section_decide(section_quadrature<256>(d1, d2, (float)(zr_ * L - zl * L), ntf_pre), dtfp, L,
+                                        ntf_times, ntf);
+        if (left == 0) {
+            ntf_out[s] = ntf;
+            dtf_out[s] = (zr_ - zl) / (1.0 * ntf);
+        }
+        list_push(lists.count + 1, lists.full, left == 1, s);
+        list_push(lists.count + 2, lists.fp64, left == 2, s);
+    }
+}
+
+// The turning-angle sum of the listed slots (tube.f90:625-657): sum |c' x c''| / |c'|^2 over
+// ntf_pre + 1 samples, the integrand in FP32 from the FP32 coefficients, the sum in FP64; one
+// warp per slot.  A result within 1e-4 of a step of ceil is left to section_fp64_kernel.
+__global__ void __launch_bounds__(256) section_kernel(const LineParam *__restrict__ lp, const int *__restrict__ slot_line,
+                                                      const double *__restrict__ cze, const double *__restrict__ Len,
+                                                      int64_t node_base, int ntf_times, int ntf_pre,
+                                                      const double *__restrict__ coe, const float *__restrict__ zstep_in,
+                                                      int *__restrict__ ntf_out, double *__restrict__ dtf_out,
+                                                      const SectionLists lists)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned n = lists.count[1], nw = (gridDim.x * blockDim.x) >> 5;
+    for (unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
+        const int64_t s = lists.full[i];
+        // lane m < 18 loads coefficient m; every lane takes the FP32 derivative coefficients by
+        // shuffles, scaled once (1, 2, 3, 4, 5 for c' and 2, 6, 12, 20 for c'')
+        const float mine = lane < 18 ? (float)coe[18 * s + lane] : 0.0f;
+        float d1[3][5], d2[3][4];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+#pragma unroll
+            for (int m = 1; m <= 5; ++m) d1[d][m - 1] = (float)m * __shfl_sync(0xffffffffu, mine, 6 * d + m);
+#pragma unroll
+            for (int m = 2; m <= 5; ++m) d2[d][m - 2] = (float)(m * (m - 1)) * __shfl_sync(0xffffffffu, mine, 6 * d + m);
+        }
+        const float zstep = zstep_in[s], z64 = 64.0f * zstep;
+        float th0 = 0.0f, th1 = 0.0f, q;
+        int tj = lane;
+        float za = zstep * (float)lane, zb = zstep * (float)(lane + 32);
+        for (; tj + 32 <= ntf_pre; tj += 64) {   // two independent samples per step
+            th0 += turning_integrand(d1, d2, za, q);
+            th1 += turning_integrand(d1, d2, zb, q);
+            za += z64;
+            zb += z64;
+        }
+        if (tj <= ntf_pre) th0 += turning_integrand(d1, d2, za, q);
+        const double sum = warp_sum((double)th0 + (double)th1);
+        if (lane == 0) {
+            const int l = slot_line[s];
+            const LineParam P = lp[l];
+            const int t = (int)(s - P.slot_off), np = P.n_sec;
+            const double *cz_line = cze + (P.node_off - node_base);
+            const double zl = cze_pl_at(cz_line, np, t), zr_ = cze_pl_at(cz_line, np, t + 1);
+            const double dtfp = (zr_ - zl) / (1.0 * ntf_pre);
+            const double xr = ntf_times * (sum * dtfp * Len[l]) / dev_pi2();
+            const double fr = xr - floor(xr);
+            const bool near_step = fmin(fr, 1.0 - fr) < 1e-4 * (xr + 1.0) || !(xr == xr);
+            if (near_step) {
+                lists.fp64[atomicAdd(lists.count + 2, 1u)] = (unsigned)s;
+            } else {
+                const int ntf = (int)ceil(xr) + 1;
+                ntf_out[s] = ntf;
+                dtf_out[s] = (zr_ - zl) / (1.0 * ntf);
+            }
+        }
+    }
+}
+
+// FP64 turning angle of the sections that fall within the FP32 rounding of a step, taken from
+// their list (a few per thousand): a fixed grid of warps strides over the list, one section per
+// warp at a time, with the reference's integrand (tube.f90:625-657) in FP64 from the stored
 // coefficients.
 __global__ void section_fp64_kernel(const LineParam *__restrict__ lp, const int *__restrict__ slot_line,
                                     const double *__restrict__ cze, const double *__restrict__ Len,
                                     int64_t node_base, int ntf_times, int ntf_pre, const double *__restrict__ coe_all,
-                                    const unsigned *__restrict__ near, int *__restrict__ ntf_out,
-                                    double *__restrict__ dtf_out)
+                                    int *__restrict__ ntf_out, double *__restrict__ dtf_out, const SectionLists lists)
 {
     const unsigned nwarps = (gridDim.x * blockDim.x) >> 5;
-    const unsigned count = near[0];
+    const unsigned count = lists.count[2];
     const int lane = threadIdx.x & 31;
     for (unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += nwarps) {
-        const int64_t warp = near[4 + i];
+        const int64_t warp = lists.fp64[i];
         const int l = slot_line[warp];
         const LineParam P = lp[l];
         const int t = (int)(warp - P.slot_off);
@@ -823,32 +965,40 @@ int centerline_setup(Ctx *c, int la, int lb, CenterlineBatch &B, BatchRecords mo
     slot_line_kernel<<<nl, 256, 0, c->stream>>>(B.lp, nl, B.slot_line);
     line_prep_kernel<<<nl, 256, 0, c->stream>>>(B.lp, nl, c->d_x, c->d_y, c->d_z, B.cze, B.ck, B.ckk, B.Len,
                                                 B.node_base);
-    c->launches += 1;
+    c->launches += 2;
     kt_end(c, km);
     const unsigned wblocks = (unsigned)((slots * 32 + 255) / 256);
     km = kt_begin(c, KT_SECTION);
-    FWT_TRY(buf_reserve(c, C.scratch[24], sizeof(unsigned) * (size_t)(slots + 4)));   // near-step list
-    unsigned *d_near = (unsigned *)C.scratch[24].p;
-    FWT_CUDA(cudaMemsetAsync(d_near, 0, sizeof(unsigned), c->stream));
-    FWT_TRY(buf_reserve(c, C.scratch[28], (sizeof(double) + sizeof(float)) * (size_t)std::max<int64_t>(slots, 1)));
-    double *d_tsum = (double *)C.scratch[28].p;
-    float *d_zstep = (float *)(d_tsum + slots);
+    // lists of undecided sections: three counters, then the three lists
+    FWT_TRY(buf_reserve(c, C.scratch[24], sizeof(unsigned) * (3 * (size_t)slots + 4)));
+    SectionLists lists;
+    lists.count = (unsigned *)C.scratch[24].p;
+    lists.fine = lists.count + 4;
+    lists.full = lists.fine + slots;
+    lists.fp64 = lists.full + slots;
+    FWT_CUDA(cudaMemsetAsync(lists.count, 0, 4 * sizeof(unsigned), c->stream));
+    FWT_TRY(buf_reserve(c, C.scratch[28], sizeof(float) * (size_t)std::max<int64_t>(slots, 1)));
+    float *d_zstep = (float *)C.scratch[28].p;
     const unsigned tblocks = (unsigned)((slots + 255) / 256);
     section_coe_kernel<<<tblocks, 256, 0, c->stream>>>(B.lp, B.slot_line, slots, c->d_x, c->d_y, c->d_z, B.cze, B.ck,
-                                                      B.ckk, B.Len, B.node_base, c->p.ntf_pre, B.coe, d_zstep);
-    section_kernel<<<wblocks, 256, 0, c->stream>>>(slots, c->p.ntf_pre, B.coe, d_zstep, d_tsum);
-    section_ntf_kernel<<<tblocks, 256, 0, c->stream>>>(B.lp, B.slot_line, slots, B.cze, B.Len, B.node_base,
-                                                      c->p.ntf_times, c->p.ntf_pre, d_tsum, B.ntf, B.dtf, d_near);
-    // a fixed grid: the list holds a few sections per thousand
-    section_fp64_kernel<<<4 * 148, 256, 0, c->stream>>>(B.lp, B.slot_line, B.cze, B.Len, B.node_base,
-                                                        c->p.ntf_times, c->p.ntf_pre, B.coe, d_near, B.ntf, B.dtf);
+                                                      B.ckk, B.Len, B.node_base, c->p.ntf_times, c->p.ntf_pre, B.coe,
+                                                      d_zstep, B.ntf, B.dtf, lists);
+    // fixed grids over the lists, no larger than the slots
+    const unsigned fblocks = (unsigned)std::min<int64_t>((slots + 127) / 128, 148 * 8);
+    section_fine_kernel<<<fblocks, 128, 0, c->stream>>>(B.lp, B.slot_line, B.cze, B.Len, B.node_base, c->p.ntf_times,
+                                                       c->p.ntf_pre, B.coe, B.ntf, B.dtf, lists);
+    const unsigned wgrid = (unsigned)std::min<int64_t>((slots + 7) / 8, 148 * 8);
+    section_kernel<<<wgrid, 256, 0, c->stream>>>(B.lp, B.slot_line, B.cze, B.Len, B.node_base, c->p.ntf_times,
+                                                 c->p.ntf_pre, B.coe, d_zstep, B.ntf, B.dtf, lists);
+    section_fp64_kernel<<<(unsigned)std::min<int64_t>((slots + 7) / 8, 4 * 148), 256, 0, c->stream>>>(
+        B.lp, B.slot_line, B.cze, B.Len, B.node_base, c->p.ntf_times, c->p.ntf_pre, B.coe, B.ntf, B.dtf, lists);
     c->launches += 4;
     kt_end(c, km);
     km = kt_begin(c, KT_CENTERLINE);
     slot_counts_kernel<<<(unsigned)((slots + 255) / 256), 256, 0, c->stream>>>(B.lp, B.slot_line, slots, B.ntf,
                                                                                B.soff, B.qoff);
     line_ntf_stats_kernel<<<nl, 256, 0, c->stream>>>(B.lp, nl, B.ntf, d_misc);
-    c->launches += 4;
+    c->launches += 2;
     FWT_CUDA(cudaGetLastError());
     FWT_TRY(scan_exclusive_i64(c, B.soff, slots, d_misc + 2 * nl, C.scratch[12]));
     FWT_TRY(scan_exclusive_i64(c, B.qoff, slots, d_misc + 2 * nl + 1, C.scratch[13]));
