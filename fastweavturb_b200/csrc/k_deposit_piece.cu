@@ -357,9 +357,8 @@ struct PBox {
     int pad[3];
 };
 
-// Rows of one chord's box (clipped to the tile in the tile kernel, whole in the scatter kernel),
-// along the axis best aligned with the chord; the box is in offsets from the piece's box origin
-// (the kernels' rx, ry, rz).
+// Rows of one chord's box (clipped to the tile) along the axis best aligned with the chord; the box
+// is in offsets from the piece's box origin (the kernels' rx, ry, rz).
 constexpr int kMaxCol = 16;   // columns, and rows per column, of a per-column row table
 struct ChordRows {          // lane-major (one entry per chord lane): conflict-free stores
     uint16_t o[3][32];      // box origin
@@ -568,23 +567,23 @@ __device__ __forceinline__ void pclip(const PieceRec &R, uint32_t img, int N, in
 // (accepted) or 2: a plane test within its rounding bound (guard) of zero, which the
 // reference's FP64 tests decide (the field jumps across the plane two consecutive chords
 // share).  The caller keeps the point in chord j's box.
-__device__ __forceinline__ int piece_classify(const PieceRec &R, int j, int rx, int ry, int rz)
+__device__ __forceinline__ int piece_classify(const PieceRec &R, int j, float rx, float ry, float rz)
 {
-    const float dxv = fmaf((float)rx, R.dx, R.off[0]);
-    const float dyv = fmaf((float)ry, R.dx, R.off[1]);
-    const float dzv = fmaf((float)rz, R.dx, R.off[2]);
+    const float dxv = fmaf(rx, R.dx, R.off[0]);
+    const float dyv = fmaf(ry, R.dx, R.off[1]);
+    const float dzv = fmaf(rz, R.dx, R.off[2]);
     const float4 p0 = R.pl[j], p1 = R.pl[j + 1];
     const float tj = fmaf(dzv, p0.z, fmaf(dyv, p0.y, fmaf(dxv, p0.x, -p0.w)));
     const float tk = fmaf(dzv, p1.z, fmaf(dyv, p1.y, fmaf(dxv, p1.x, -p1.w)));
-    if (!(tj >= -R.guard) || !(tk < R.guard)) return 0;
     const float4 cp = R.po[j];
-    const float ex = fmaf((float)rx, R.dx, cp.x);
-    const float ey = fmaf((float)ry, R.dx, cp.y);
-    const float ez = fmaf((float)rz, R.dx, cp.z);
+    const float ex = fmaf(rx, R.dx, cp.x);
+    const float ey = fmaf(ry, R.dx, cp.y);
+    const float ez = fmaf(rz, R.dx, cp.z);
     const float t0 = fmaf(ez, p0.z, fmaf(ey, p0.y, ex * p0.x));
     const float r2 = fmaf(-t0, t0, fmaf(ez, ez, fmaf(ey, ey, ex * ex)));
-    if (!(r2 < R.chq[j].y)) return 0;
-    return (tj >= R.guard && tk < -R.guard) ? 1 : 2;
+    const bool in = (tj >= -R.guard) & (tk < R.guard) & (r2 < R.chq[j].y);
+    const bool sure = (tj >= R.guard) & (tk < -R.guard);
+    return in ? (sure ? 1 : 2) : 0;
 }
 
 // The candidate test of the FP64 path: piece_classify with every test widened by far more than
@@ -1022,122 +1021,226 @@ __global__ void __launch_bounds__(kDepThreads, F64 ? 2 : 3) deposit_piece_kernel
 // Thin tubes without tiles.  The tile kernels pay, for every (tile, piece) pair, a record copy
 // and every chord's set-up within that tile; a thin chord accepts a few points and its box
 // meets two to six tiles, so that overhead outweighs the evaluations.  The scatter kernel takes
-// each piece once: a warp stages kPChunk pieces (32 chords, one per lane), each lane builds its
-// chord's row table over the chord's whole box (chord_row_table), the rows are spread over the
-// lanes (chord_row_span), their candidates tested 32 at a time (piece_classify) and the accepted
-// pairs evaluated 32 at a time; each contribution is added as int64 fixed point into the side
-// accumulator with global reductions.  Integer sums do not depend on the order, so the field is
-// deterministic; side_fold adds the sums into omega after the batch loop.  Pairs for the FP64
-// tests or arithmetic are deferred as in the tile kernels.
+// each piece once: a warp stages kPChunk pieces (32 chords, one per lane); each lane works out its
+// chord's rows (chord_rows); four or eight lanes then take a chord's rows each, and queue the
+// points of the index intervals that the rows can accept; candidates are tested 32 at a time
+// (piece_classify) and the accepted pairs evaluated 32 at a time; each contribution is added as
+// int64 fixed point into the side accumulator with global reductions.  Integer sums do not
+// depend on the order, so the field is deterministic; side_fold adds the sums into omega after
+// the batch loop.  Pairs for the FP64 tests or arithmetic are deferred as in the tile kernels.
+//
+// Bound by instruction issue (73 % of the slots, 4,300 instructions for 28 chords of radius 1.9)
+// while the sums stay within the L2, and by the reductions' trips to HBM beyond: 64 bytes a pair
+// at 2.9 TB/s.  512 tubes of 4096 nodes on 512^3, ms without side_fold, against rows listed along
+// the best-aligned axis inside the chord's ellipse, found by binary search, and three reductions
+// a pair: radius 1.9: 5.7 -> 4.9, 3.8: 38.3 -> 24.4, 7.6: 306 -> 202.
+//   - Rows run along the axis that gives the fewest of them: a chord is a disk about as thick as
+//     a spacing, and rows within its plane hold several points, rows across it mostly none.  x is
+//     preferred, where a row's sums are contiguous.
+//   - The bounds of a row are linear in its offsets, so that a row costs two fused multiply-adds a
+//     bound and one square root; a rectangle of rows needs no list and no search.
+//   - Four lanes add a pair's three sums as one 32-byte sector: 140-210 G pairs/s where three
+//     reductions of one lane each ran at 55-73.
+//   - Fewer registers and a fourth block per SM were slower (3.8: 32 -> 33.5 ms).
 constexpr int kScatterWarps = 8;
 constexpr uint32_t kSQDecide = 1u << 31;     // queued pair left to the reference's FP64 tests
 struct ScatterStage {
     PieceRec rec[kPChunk];
-    ChordRows cr;
-    uint32_t cq[kPQueue];   // candidates: chord lane | x << 5 | y << 13 | z << 21 (offsets from the piece's box origin)
-    uint32_t q[kPQueue];    // accepted pairs: the same | kSQDecide
+    float4 lo[32], hi[32];      // chord lane: bounds A + B rb + C rc of a row's index, and the box's bound
+    float4 dist[32], mid[32];   // cylinder: (D0, Db, Dc, R^2) and (M0, Mb, Mc, 1 / (1 - n_a^2))
+    float4 box[32];             // rows along b: (n, 1 / n, code of the first row), rows in all
+    uint32_t sel[32];           // byte order that turns (b, c, a) offsets into (x, y, z)
+    uint32_t cq[128];           // candidates: x | y << 8 | z << 16 | chord lane << 24 (offsets from the piece's box origin)
+    uint32_t q[64];             // accepted pairs: the same | kSQDecide
+    longlong2 sum[64];            // contributions: three int64, and the cell (-1: none)
 };
 constexpr size_t kScatterSmem = sizeof(ScatterStage) * kScatterWarps;
+static_assert(3 * (kScatterSmem + 1024) <= 228 * 1024, "scatter_piece_kernel: three blocks per SM");
 
-// Test the first cnt candidates (piece_classify), queue the accepted pairs and those left to
-// the FP64 tests, and drop the candidates.
-__device__ __forceinline__ void scatter_test(ScatterStage &S, int lane, int cnt, int &cn, int &qn)
+// Byte i of v as a float (0..255), without the conversion unit.
+template <int I>
+__device__ __forceinline__ float byte_float(uint32_t v)
 {
-    bool ok = false;
-    uint32_t code = 0u;
-    if (lane < cnt) {
-        const uint32_t e = S.cq[lane];
-        const int c = (int)(e & 31u);
-        const int cls = piece_classify(S.rec[c >> 3], c & 7, (int)((e >> 5) & 255u), (int)((e >> 13) & 255u),
-                                       (int)((e >> 21) & 255u));
-        ok = cls != 0;
-        code = e | (cls == 2 ? kSQDecide : 0u);
+    return __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440u + I)) - 8388608.0f;
+}
+__device__ __forceinline__ float comp3(int d, float x, float y, float z) { return d == 0 ? x : (d == 1 ? y : z); }
+
+// Rounding to an integer in the low mantissa bits: bits(v + kMagic) - bits(kMagic) = rint(v).  A
+// lower bound v becomes the first index rint(v + 0.44) <= ceil(v), an upper bound the last index
+// rint(v - 0.44) >= floor(v): indices within 0.06 of the bound stay in.
+constexpr float kMagic = 12582912.0f;
+
+// Row geometry of chord j (lane's chord) over its whole box [co, co + cnn).  A row is a line of mesh
+// points along axis a; the chord's rows fill a rectangle of offsets (rb, rc) along the other two
+// axes, and the indices that a row can accept are bounded by linear forms of (rb, rc).  All lengths
+// in grid spacings, offsets from the piece's box origin.
+//   Axis: the one least aligned with the chord whose rows both planes still bound (|n_a| >= 0.15),
+//   x before the others; the best aligned one where none is.
+//   Rectangle: the accepted points S_j + t n + v, |v| < Rtube, v . n = 0, 0 <= t < l + Rtube tan(theta)
+//   (theta: the angle between the planes; plane j + 1 passes through S_j + l n) reach
+//   Rtube sqrt(1 - n_b^2) along b on either side of the sweep.
+//   Planes: t_j >= -guard and t_{j+1} < guard (a plane nearly parallel to the rows, or facing the
+//   other way, gives no bound).
+//   Cylinder: the row passes the chord's line at distance D, next to index m, and stays within
+//   Rtube of it for sqrt((Rtube^2 - D^2) / (1 - n_a^2)) on either side.
+__device__ __forceinline__ void chord_rows(const PieceRec &R, int j, const int co[3], const int cnn[3], ScatterStage &S,
+                                           int lane)
+{
+    const float4 pj = R.pl[j], pk = R.pl[j + 1], oj = R.po[j], ok1 = R.po[j + 1];
+    const float ax = fabsf(pj.x), ay = fabsf(pj.y), az = fabsf(pj.z);
+    const float kx = ax >= 0.15f && pk.x * pj.x >= 0.1f * ax ? ax - 0.3f : 4.0f - ax;
+    const float ky = ay >= 0.15f && pk.y * pj.y >= 0.1f * ay ? ay : 4.0f - ay;
+    const float kz = az >= 0.15f && pk.z * pj.z >= 0.1f * az ? az : 4.0f - az;
+    const int a = (kx <= ky && kx <= kz) ? 0 : (ky <= kz ? 1 : 2);
+    const int b = a == 0 ? 1 : 0, c = a == 2 ? 1 : 2;
+    S.sel[lane] = a == 0 ? 0x3104u : (a == 1 ? 0x3140u : 0x3410u);
+    const float idx = __fdividef(1.0f, R.dx);
+    const float na = comp3(a, pj.x, pj.y, pj.z), nb = comp3(b, pj.x, pj.y, pj.z), nc = comp3(c, pj.x, pj.y, pj.z);
+    const float ma = comp3(a, pk.x, pk.y, pk.z), mb = comp3(b, pk.x, pk.y, pk.z), mc = comp3(c, pk.x, pk.y, pk.z);
+    const int oa = a == 0 ? co[0] : (a == 1 ? co[1] : co[2]);
+    const int ea = a == 0 ? cnn[0] : (a == 1 ? cnn[1] : cnn[2]), eb = b == 0 ? cnn[0] : (b == 1 ? cnn[1] : cnn[2]),
+              ec = c == 0 ? cnn[0] : (c == 1 ? cnn[1] : cnn[2]);
+    // the chord's start and the rectangle
+    const float sa = -idx * comp3(a, oj.x, oj.y, oj.z), sb = -idx * comp3(b, oj.x, oj.y, oj.z),
+                sc = -idx * comp3(c, oj.x, oj.y, oj.z);
+    const float rt = sqrtf(R.chq[j].y) * idx;
+    float b0 = (float)(b == 0 ? co[0] : (b == 1 ? co[1] : co[2])), b1 = b0 + (float)(eb - 1);
+    float c0 = (float)(c == 0 ? co[0] : (c == 1 ? co[1] : co[2])), c1 = c0 + (float)(ec - 1);
+    const float cth = pj.x * pk.x + pj.y * pk.y + pj.z * pk.z;
+    if (cth > 0.5f) {
+        const float lx = oj.x - ok1.x, ly = oj.y - ok1.y, lz = oj.z - ok1.z;
+        const float sweep = sqrtf(lx * lx + ly * ly + lz * lz) * idx +
+                            __fdividef(rt * sqrtf(fmaxf(1.0f - cth * cth, 0.0f)), cth);
+        const float tb = sweep * nb, tc = sweep * nc;
+        const float hb = fmaf(rt * sqrtf(fmaxf(1.0f - nb * nb, 0.0f)), 1.001f, 0.02f),
+                    hc = fmaf(rt * sqrtf(fmaxf(1.0f - nc * nc, 0.0f)), 1.001f, 0.02f);
+        b0 = ((fmaxf(b0, sb + fminf(tb, 0.0f) - hb) + 0.44f) + kMagic) - kMagic;
+        b1 = ((fminf(b1, sb + fmaxf(tb, 0.0f) + hb) - 0.44f) + kMagic) - kMagic;
+        c0 = ((fmaxf(c0, sc + fminf(tc, 0.0f) - hc) + 0.44f) + kMagic) - kMagic;
+        c1 = ((fminf(c1, sc + fmaxf(tc, 0.0f) + hc) - 0.44f) + kMagic) - kMagic;
     }
-    const unsigned bal = __ballot_sync(0xffffffffu, ok);
-    if (ok) S.q[qn + __popc(bal & ((1u << lane) - 1u))] = code;
-    qn += __popc(bal);
-    const int rem = cn - cnt;
-    const uint32_t keep = lane < rem ? S.cq[cnt + lane] : 0u;
-    __syncwarp();
-    if (lane < rem) S.cq[lane] = keep;
-    __syncwarp();
-    cn = rem;
+    const float nbf = b1 - b0 + 1.0f, ncf = c1 - c0 + 1.0f;
+    const bool any = nbf > 0.5f && ncf > 0.5f;
+    const uint32_t code = any ? (uint32_t)b0 | ((uint32_t)c0 << 8) | ((uint32_t)lane << 24) : 0u;
+    S.box[lane] = make_float4(any ? nbf : 1.0f, any ? __fdividef(1.0f, nbf) : 1.0f, __uint_as_float(code),
+                              any ? nbf * ncf : 0.0f);
+    // planes, at (rb, rc) from the rectangle's corner
+    const float g = R.guard * idx;
+    const float ina = __fdividef(1.0f, na), ima = __fdividef(1.0f, ma);
+    const float dj = (pj.x * oj.x + pj.y * oj.y + pj.z * oj.z) * idx + fmaf(nb, b0, nc * c0);
+    const float dk = (pk.x * ok1.x + pk.y * ok1.y + pk.z * ok1.z) * idx + fmaf(mb, b0, mc * c0);
+    const bool up = na > 0.0f;   // t_j grows with the index
+    const bool both = up ? ma > 0.05f : ma < -0.05f;
+    const float g0 = fabsf(g * ina), g1 = both ? fabsf(g * ima) : 0.0f;
+    const float4 F0 = make_float4(-dj * ina + (up ? -g0 : g0), -nb * ina, -nc * ina, 0.0f);
+    const float4 F1 = both ? make_float4(-dk * ima + (up ? g1 : -g1), -mb * ima, -mc * ima, 0.0f)
+                           : make_float4(up ? 1.0e9f : -1.0e9f, 0.0f, 0.0f, 0.0f);
+    float4 L = up ? F0 : F1, H = up ? F1 : F0;
+    L.w = (float)oa;
+    H.w = (float)(oa + ea - 1);
+    S.lo[lane] = L;
+    S.hi[lane] = H;
+    // cylinder (none where the rows are nearly parallel to the chord)
+    const float nbc2 = 1.0f - na * na;
+    const bool bound = nbc2 > 0.01f;
+    const float inbc = bound ? rsqrt_hw(nbc2) : 0.0f, iq = bound ? inbc * inbc : 1.0f;
+    const float wb = nb * inbc, wc = nc * inbc, r = fmaf(rt, 1.001f, 0.02f);
+    S.dist[lane] = make_float4(wc * (sb - b0) - wb * (sc - c0), -wc, wb, bound ? r * r : 1.0e12f);
+    const float ki = bound ? na * iq : 0.0f;
+    S.mid[lane] = make_float4(sa - ki * (nb * (sb - b0) + nc * (sc - c0)), ki * nb, ki * nc, iq);
 }
 
-// Evaluate the first cnt queued pairs, one per lane, and add them into the side accumulator;
+// Test the last cnt candidates (piece_classify) and queue the accepted pairs and those left to
+// the FP64 tests.  Lanes beyond cnt test whatever they find (in bounds) and drop it.
+__device__ __forceinline__ void scatter_test(ScatterStage &S, int lane, int cnt, int &cn, int &qn)
+{
+    cn -= cnt;
+    const uint32_t e = S.cq[cn + lane];
+    const int c = (int)(e >> 24) & 31;
+    const int cls = piece_classify(S.rec[c >> 3], c & 7, byte_float<0>(e), byte_float<1>(e), byte_float<2>(e));
+    const bool ok = cls != 0 && lane < cnt;
+    const unsigned bal = __ballot_sync(0xffffffffu, ok);
+    if (ok) S.q[qn + __popc(bal & ((1u << lane) - 1u))] = cls == 2 ? e | kSQDecide : e;
+    qn += __popc(bal);
+    __syncwarp();
+}
+
+// Evaluate the last cnt queued pairs, one per lane, and add them into the side accumulator;
 // the pairs left to FP64 (kSQDecide, or a curved-branch amplification above kRedoCond) are
-// deferred.  Points outside the context's planes (a z-slab context) are dropped.
+// deferred.  Points outside the context's planes (a z-slab context) are dropped, and so is what
+// the lanes beyond cnt computed.  With prefetch (sums beyond the L2) the cell is asked for before the
+// vorticity is computed: a reduction that misses the L2 holds the queue up (512^3, truncation radius
+// 3.8 spacings: 13.5 -> 12.4 ms; sums within the L2, 128^3: 12.5 -> 12.6, so not there).
 template <bool General>
 __device__ __forceinline__ void scatter_drain(ScatterStage &S, int lane, int cnt, int &qn, int64_t p0, int N, int zs,
                                               int nz, float fscale, unsigned long long *__restrict__ side,
-                                              int *__restrict__ err, const DeferList &D, unsigned long long &nacc)
+                                              bool prefetch, int *__restrict__ err, const DeferList &D, unsigned long long &nacc)
 {
-    bool flag = false, counted = false;
-    uint32_t rrec = 0;
-    int gx = 0, gy = 0, gz = 0;
-    if (lane < cnt) {
-        const uint32_t e = S.q[lane];
-        const int c = (int)(e & 31u), k = c >> 3, j = c & 7;
-        const int rx = (int)((e >> 5) & 255u), ry = (int)((e >> 13) & 255u), rz = (int)((e >> 21) & 255u);
-        const PieceRec &R = S.rec[k];
-        // unwrapped 0-based indices lie within one period of the domain (checked with the chord
-        // boxes): one conditional shift wraps them, no integer division
-        gx = R.box_lo[0] - 1 + rx;
-        gy = R.box_lo[1] - 1 + ry;
-        gz = R.box_lo[2] - 1 + rz;
-        gx += gx < 0 ? N : (gx >= N ? -N : 0);
-        gy += gy < 0 ? N : (gy >= N ? -N : 0);
-        gz += gz < 0 ? N : (gz >= N ? -N : 0);
-        const bool inslab = gz >= zs && gz < zs + nz;
-        const uint32_t id = ((uint32_t)(p0 + k) & ((1u << 26) - 1u)) | ((uint32_t)j << 26);
-        if (inslab && (e & kSQDecide)) {
-            flag = true;
-            rrec = id | kDeferDecide;
-        } else if (inslab && (General || !D.emit_only)) {
-            counted = true;
-            const float4 cp = R.po[j], cq = R.chq[j], pn = R.pl[j];
-            const float ex = fmaf((float)rx, R.dx, cp.x);
-            const float ey = fmaf((float)ry, R.dx, cp.y);
-            const float ez = fmaf((float)rz, R.dx, cp.z);
-            const float t0 = fmaf(ez, pn.z, fmaf(ey, pn.y, ex * pn.x));
-            float vv[3], cond;
-            vort_w<General, true>(R, ex, ey, ez, cp.w, t0 * cq.x, cq.y, vv, cond);
-            flag = General && !(cond <= kRedoCond);
-            if (flag) {
-                rrec = id;
-            } else if (!D.emit_only) {
-                const size_t g = (size_t)gx + (size_t)N * ((size_t)gy + (size_t)N * (size_t)(gz - zs));
+    qn -= cnt;
+    const uint32_t e = S.q[qn + lane];
+    const int c = (int)((e >> 24) & 31u), k = c >> 3, j = c & 7;
+    const PieceRec &R = S.rec[k];
+    // unwrapped 0-based indices lie within one period of the domain (checked with the chord
+    // boxes): one conditional shift wraps them, no integer division
+    int gx = R.box_lo[0] - 1 + (int)(e & 255u);
+    int gy = R.box_lo[1] - 1 + (int)((e >> 8) & 255u);
+    int gz = R.box_lo[2] - 1 + (int)((e >> 16) & 255u);
+    gx += gx < 0 ? N : (gx >= N ? -N : 0);
+    gy += gy < 0 ? N : (gy >= N ? -N : 0);
+    gz += gz < 0 ? N : (gz >= N ? -N : 0);
+    const bool inslab = lane < cnt && gz >= zs && gz < zs + nz;
+    const long long cell = (long long)gx + (long long)N * ((long long)gy + (long long)N * (long long)(gz - zs));
+    if (prefetch && inslab) asm volatile("prefetch.global.L2 [%0];" ::"l"(side + kSideStride * cell));
+    const bool decide = (e & kSQDecide) != 0u;
+    const bool counted = inslab && !decide && (General || !D.emit_only);
+    const float4 cp = R.po[j], cq = R.chq[j], pn = R.pl[j];
+    const float ex = fmaf(byte_float<0>(e), R.dx, cp.x);
+    const float ey = fmaf(byte_float<1>(e), R.dx, cp.y);
+    const float ez = fmaf(byte_float<2>(e), R.dx, cp.z);
+    const float t0 = fmaf(ez, pn.z, fmaf(ey, pn.y, ex * pn.x));
+    float vv[3], cond;
+    vort_w<General, true>(R, ex, ey, ez, cp.w, t0 * cq.x, cq.y, vv, cond);
+    const bool redo = General && counted && !(cond <= kRedoCond);
+    const bool add = counted && !redo && !D.emit_only;
+    const float sv[3] = {vv[0] * fscale, vv[1] * fscale, vv[2] * fscale};
+    long long sum[3];
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    float sv = vv[d] * fscale;
-                    if (!(fabsf(sv) < 4.0e18f)) {
-                        atomicOr(err, 4);
-                        sv = sv != sv ? 0.0f : copysignf(4.0e18f, sv);
-                    }
-                    atomicAdd(side + kSideStride * g + d, (unsigned long long)__float2ll_rn(sv));
-                }
+    for (int d = 0; d < 3; ++d) sum[d] = __float2ll_rn(sv[d]);
+    // (the sum is NaN or infinite where a component is)
+    if (add && !(fabsf(sv[0]) + fabsf(sv[1]) + fabsf(sv[2]) < 4.0e18f)) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+            if (!(fabsf(sv[d]) < 4.0e18f)) {
+                atomicOr(err, 4);
+                sum[d] = sv[d] != sv[d] ? 0 : __float2ll_rn(copysignf(4.0e18f, sv[d]));
             }
-        }
+    }
+    // four lanes to a cell (three of them add): a reduction's 32-byte sector goes out once, not
+    // three times
+    S.sum[2 * lane] = longlong2{sum[0], sum[1]};
+    S.sum[2 * lane + 1] = longlong2{sum[2], add ? cell : -1};
+    __syncwarp();
+    const long long *flat = reinterpret_cast<const long long *>(S.sum);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const long long v = flat[32 * i + lane], g = flat[32 * i + (lane | 3)];
+        if (g >= 0 && (lane & 3) < 3) atomicAdd(side + kSideStride * g + (lane & 3), (unsigned long long)v);
     }
     nacc += (unsigned long long)__popc(__ballot_sync(0xffffffffu, counted));
-    defer_push(D, lane, flag, rrec, gx, gy, gz);
+    const uint32_t id = ((uint32_t)(p0 + k) & ((1u << 26) - 1u)) | ((uint32_t)j << 26);
+    defer_push(D, lane, redo || (inslab && decide), decide ? id | kDeferDecide : id, gx, gy, gz);
     __syncwarp();
-    const int rem = qn - cnt;
-    const uint32_t keep = lane < rem ? S.q[cnt + lane] : 0u;
-    __syncwarp();
-    if (lane < rem) S.q[lane] = keep;
-    __syncwarp();
-    qn = rem;
 }
 
 template <bool General>
 __global__ void __launch_bounds__(kScatterWarps * 32, 3) scatter_piece_kernel(
     const PieceRec *__restrict__ rec, int64_t npieces, int N, int zs, int nz, float fscale,
-    unsigned long long *__restrict__ side, int *__restrict__ err, const DeferList D,
+    unsigned long long *__restrict__ side, int prefetch, int *__restrict__ err, const DeferList D,
     unsigned long long *__restrict__ tally)
 {
     extern __shared__ __align__(16) unsigned char dsm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
     ScatterStage &S = reinterpret_cast<ScatterStage *>(dsm)[warp];
     const int64_t nchunks = (npieces + kPChunk - 1) / kPChunk;
     const int64_t nw = (int64_t)gridDim.x * kScatterWarps;
@@ -1153,8 +1256,8 @@ __global__ void __launch_bounds__(kScatterWarps * 32, 3) scatter_piece_kernel(
             for (int t = lane; t < n16; t += 32) dst[t] = __ldg(src + t);
         }
         __syncwarp();
-        // lane = (piece k, chord j): the chord's whole box and its rows
-        int nrows = 0;
+        // lane = (piece k, chord j): the chord's whole box, its rows' bounds and its columns
+        S.box[lane] = make_float4(1.0f, 1.0f, 0.0f, 0.0f);   // no rows
         {
             const int k = lane >> 3, j = lane & 7;
             if (k < nc && j < S.rec[k].nch) {
@@ -1176,54 +1279,63 @@ __global__ void __launch_bounds__(kScatterWarps * 32, 3) scatter_piece_kernel(
                     atomicOr(err, 64);
                     nonempty = false;
                 }
-                nrows = chord_row_table(R, j, co, cnn, nonempty, S.cr, lane);
+                if (nonempty) chord_rows(R, j, co, cnn, S, lane);
             }
         }
-        int incl = nrows;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const int roff = incl - nrows;
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
         __syncwarp();
         int cn = 0, qn = 0;   // queued candidates and pairs (warp-uniform)
-        for (int r0 = 0; r0 < total; r0 += 32) {
-            const int r = r0 + lane;
-            int c = 0;   // chord lane of row r: last lane whose first row is <= r
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1) {
-                const int t = c + step;
-                const int ot = __shfl_sync(0xffffffffu, roff, t);
-                if (ot <= r) c = t;
-            }
-            const int rc = __shfl_sync(0xffffffffu, roff, c);
-            int i = 1, ihi = 0, a = 0, bx = 0, by = 0, bz = 0;
-            if (r < total) chord_row_span(S.rec[c >> 3], S.cr, c, c & 7, r - rc, bx, by, bz, a, i, ihi);
-            while (__any_sync(0xffffffffu, i <= ihi)) {
-                const bool has = i <= ihi;
-                uint32_t code = 0u;
-                if (has) {
-                    code = (uint32_t)c | ((uint32_t)(bx + (a == 0 ? i : 0)) << 5) |
-                           ((uint32_t)(by + (a == 1 ? i : 0)) << 13) | ((uint32_t)(bz + (a == 2 ? i : 0)) << 21);
-                    ++i;
-                }
-                const unsigned bal = __ballot_sync(0xffffffffu, has);
-                if (has) S.cq[cn + __popc(bal & ((1u << lane) - 1u))] = code;
-                cn += __popc(bal);
-                __syncwarp();
-                if (cn >= 32) {
-                    scatter_test(S, lane, 32, cn, qn);
-                    if (qn >= 32) scatter_drain<General>(S, lane, 32, qn, p0, N, zs, nz, fscale, side, err, D, nacc);
-                }
+        // chord after chord, so that 32 consecutive candidates (and pairs from them) read few
+        // different records: four lanes to a chord of at most 16 rows, eight to a larger one (radius
+        // 1.5: 7.6 and 8.5 ms, 3.8: 31.4 and 29.0)
+        const int ls = __reduce_max_sync(0xffffffffu, __float_as_int(S.box[lane].w)) <= __float_as_int(16.0f) ? 2 : 3;
+        const float l0 = (float)(lane & ((1 << ls) - 1)), lstep = (float)(1 << ls);
+        for (int c0 = 0; c0 < 8 * nc; c0 += 32 >> ls) {
+            const int c = c0 + (lane >> ls);
+            const float rows = S.box[c].w;
+            for (float row = l0; __any_sync(0xffffffffu, row < rows); row += lstep) {
+                // the interval of indices the lane's row can accept
+                const float4 B = S.box[c], L = S.lo[c], H = S.hi[c], Q = S.dist[c], M = S.mid[c];
+                const uint32_t sel = S.sel[c];
+                const float tc = fmaf(row, B.y, fmaf(0.5f, B.y, -0.5f)) + kMagic, rc = tc - kMagic;
+                const float rb = fmaf(-B.x, rc, row);
+                const uint32_t rcode = __float_as_uint(B.z) + (__byte_perm(__float_as_uint(rb + kMagic),
+                                                                          __float_as_uint(tc), 0x40u) & 0xffffu);
+                const float D0 = fmaf(Q.z, rc, fmaf(Q.y, rb, Q.x));
+                const float q = fmaf(-D0, D0, Q.w) * M.w;
+                const float m = fmaf(M.z, rc, fmaf(M.y, rb, M.x));
+                float h;
+                asm("sqrt.approx.f32 %0, %1;" : "=f"(h) : "f"(fmaxf(q, 0.0f)));
+                const float lo = fmaxf(fmaxf(fmaf(L.z, rc, fmaf(L.y, rb, L.x)), L.w), m - h);
+                const float hi = fminf(fminf(fmaf(H.z, rc, fmaf(H.y, rb, H.x)), H.w), m + h);
+                uint32_t i = __float_as_uint((fminf(lo, 1000.0f) + 0.44f) + kMagic);
+                int n_ = __float_as_int((fmaxf(hi, -1000.0f) - 0.44f) + kMagic) - (int)i + 1;
+                if (row >= rows || q < 0.0f) n_ = 0;
+                bool left;
+                do {
+                    // up to three candidates a row, counted with two ballots
+                    const int m = min(max(n_, 0), 3);
+                    const unsigned m1 = __ballot_sync(0xffffffffu, m & 1), m2 = __ballot_sync(0xffffffffu, m & 2);
+                    uint32_t *dst = S.cq + cn + __popc(m1 & below) + 2 * __popc(m2 & below);
+                    if (m > 0) dst[0] = __byte_perm(rcode, i, sel);
+                    if (m > 1) dst[1] = __byte_perm(rcode, i + 1u, sel);
+                    if (m > 2) dst[2] = __byte_perm(rcode, i + 2u, sel);
+                    cn += __popc(m1) + 2 * __popc(m2);
+                    i += 3u;
+                    n_ -= 3;
+                    left = __any_sync(0xffffffffu, n_ > 0);
+                    __syncwarp();
+                    while (cn >= 32) {
+                        scatter_test(S, lane, 32, cn, qn);
+                        if (qn >= 32) scatter_drain<General>(S, lane, 32, qn, p0, N, zs, nz, fscale, side, prefetch, err, D, nacc);
+                    }
+                } while (left);
             }
         }
-        while (cn > 0) {
-            scatter_test(S, lane, min(cn, 32), cn, qn);
-            if (qn >= 32) scatter_drain<General>(S, lane, 32, qn, p0, N, zs, nz, fscale, side, err, D, nacc);
+        if (cn > 0) {
+            scatter_test(S, lane, cn, cn, qn);
+            if (qn >= 32) scatter_drain<General>(S, lane, 32, qn, p0, N, zs, nz, fscale, side, prefetch, err, D, nacc);
         }
-        while (qn > 0) scatter_drain<General>(S, lane, min(qn, 32), qn, p0, N, zs, nz, fscale, side, err, D, nacc);
+        if (qn > 0) scatter_drain<General>(S, lane, qn, qn, p0, N, zs, nz, fscale, side, prefetch, err, D, nacc);
         __syncwarp();   // the warp's stage is reused by its next chunk
     }
     if (lane == 0 && tally && !D.emit_only && nacc) atomicAdd(tally, nacc);
@@ -1449,6 +1561,10 @@ int launch_scatter(Ctx *c, const CenterlineBatch &B)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
     const int64_t nchunks = (B.npieces + kPChunk - 1) / kPChunk;
     unsigned long long *side = (unsigned long long *)c->b_side.p;
+    // sums beyond the L2: fetched ahead of their additions (see scatter_drain)
+    int l2 = 0;
+    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c->dev);
+    const int prefetch = sizeof(long long) * kSideStride * (size_t)N * N * nz > (size_t)l2;
     DeferList D{};
     FWT_TRY(defer_list(c, B.npieces, c->defer_per_piece, D));
     auto launch = [&](const DeferList &L) -> int {
@@ -1459,12 +1575,12 @@ int launch_scatter(Ctx *c, const CenterlineBatch &B)
             FWT_CUDA(cudaFuncSetAttribute(scatter_piece_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)kScatterSmem));
             scatter_piece_kernel<true><<<grid, kScatterWarps * 32, kScatterSmem, c->stream>>>(
-                B.piece, B.npieces, N, zs, nz, (float)scale, side, d_err, L, rctx.tally);
+                B.piece, B.npieces, N, zs, nz, (float)scale, side, prefetch, d_err, L, rctx.tally);
         } else {
             FWT_CUDA(cudaFuncSetAttribute(scatter_piece_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)kScatterSmem));
             scatter_piece_kernel<false><<<grid, kScatterWarps * 32, kScatterSmem, c->stream>>>(
-                B.piece, B.npieces, N, zs, nz, (float)scale, side, d_err, L, rctx.tally);
+                B.piece, B.npieces, N, zs, nz, (float)scale, side, prefetch, d_err, L, rctx.tally);
         }
         FWT_CUDA(cudaGetLastError());
         kt_end(c, m);
