@@ -277,6 +277,9 @@ int fwt_destroy(fwt_ctx *h)
     }
     for (auto &p : c->fbb_plans) cufftDestroy(p.h);
     c->fbb_plans.clear();
+    if (c->fbb_ws) cudaFree(c->fbb_ws);
+    c->fbb_ws = nullptr;
+    c->fbb_ws_bytes = 0;
     buf_free(c, c->b_nodes);
     buf_free(c, c->b_w);
     buf_free(c, c->b_u);

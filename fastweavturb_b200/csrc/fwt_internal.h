@@ -106,12 +106,16 @@ struct Ctx {
     DevBuf b_aux_spec, b_aux_real, b_aux_acc, b_aux_out;   // their buffers, made on first use
     cufftHandle plan_r2c = 0, plan_c2r = 0;
     // the generator's plans, kept between calls (plan creation costs milliseconds and a device
-    // synchronisation): key n2 for the single circulant row (batch 0) or (n2, batch)
+    // synchronisation): key n2 for the single circulant row (batch 0) or (n2, batch).  They run one
+    // after the other on the context's stream and share one work area, the largest any of them needs
     struct FftPlan {
         int n2, batch;
         cufftHandle h;
+        size_t ws;
     };
     std::vector<FftPlan> fbb_plans;
+    void *fbb_ws = nullptr;
+    size_t fbb_ws_bytes = 0;
     bool plans = false;
     size_t fft_ws_bytes = 0;
 

@@ -51,11 +51,18 @@ __global__ void fbb_row_kernel(int M, double H, cufftDoubleComplex *row)
     row[k].y = 0.0;
 }
 
-__global__ void fbb_sqrt_kernel(int n2, const cufftDoubleComplex *lam, double *sq)
+// square roots of the eigenvalues, and the bridge's function f(j + 1), j = 0..Np-1 (Np <= n2), which
+// all tubes of the level share, in place of the imaginary parts (two FP64 powers a node: taken per tube
+// and pass they were most of fbb_bridge_kernel)
+__global__ void fbb_sqrt_kernel(int n2, int Np, double H, cufftDoubleComplex *lam, double *sq)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n2) return;
     sq[k] = sqrt(fmax(lam[k].x, 0.0) / n2);
+    if (k < Np) {
+        const double x = (double)(k + 1) / Np;
+        lam[k].y = 0.5 * (pow(x, 2.0 * H) + 1.0 - pow(1.0 - x, 2.0 * H));
+    }
 }
 
 // Z[b][k] = sq[k] (Za + i Zb), b = 3*(tube - t0) + coord
@@ -116,7 +123,8 @@ __global__ void fbb_scan_kernel(const cufftDoubleComplex *__restrict__ W, int n2
 }
 
 // per tube: subsample (Np < 128), bridge, rms normalisation, shift, wrap
-__global__ void fbb_bridge_kernel(uint64_t seed, int t0, int Np, int M, double H, double dB,
+__global__ void fbb_bridge_kernel(uint64_t seed, int t0, int Np, int M, double dB,
+                                  const cufftDoubleComplex *__restrict__ bridge,
                                   const double *__restrict__ fbm, double *__restrict__ X, double *__restrict__ Y,
                                   double *__restrict__ Z, int64_t node0)
 {
@@ -131,16 +139,12 @@ __global__ void fbb_bridge_kernel(uint64_t seed, int t0, int Np, int M, double H
         }
         return f[co][j];
     };
-    auto fb = [&](int j) -> double {   // f_bridge(j+1)
-        const double x = (double)(j + 1) / Np;
-        return 0.5 * (pow(x, 2.0 * H) + 1.0 - pow(1.0 - x, 2.0 * H));
-    };
     double end[3];
     for (int co = 0; co < 3; ++co) end[co] = src(co, Np - 1);
     // rms of steps over the three coordinates
     double acc = 0.0;
     for (int j = threadIdx.x; j < Np - 1; j += blockDim.x) {
-        const double f0 = fb(j), f1 = fb(j + 1);
+        const double f0 = bridge[j].y, f1 = bridge[j + 1].y;
         for (int co = 0; co < 3; ++co) {
             const double d = (src(co, j + 1) - f1 * end[co]) - (src(co, j) - f0 * end[co]);
             acc += d * d / (Np - 1);
@@ -167,7 +171,7 @@ __global__ void fbb_bridge_kernel(uint64_t seed, int t0, int Np, int M, double H
     double *out[3] = {X, Y, Z};
     const int64_t o = node0 + (int64_t)tl * Np;
     for (int j = threadIdx.x; j < Np; j += blockDim.x) {
-        const double fj = fb(j);
+        const double fj = bridge[j].y;
         for (int co = 0; co < 3; ++co) {
             double v = (src(co, j) - fj * end[co]) * s_scale + s_shift[co];
             // mod(v, 2pi) - pi with MATLAB's floored modulo
@@ -177,25 +181,45 @@ __global__ void fbb_bridge_kernel(uint64_t seed, int t0, int Np, int M, double H
     }
 }
 
-// A Z2Z plan of length n2 over `batch` contiguous rows, made once per context and shape (at
-// most eight are kept; the oldest is dropped).
+// A Z2Z plan of length n2 over `batch` contiguous rows, made once per context and shape.  A level
+// takes two (its circulant row and its tubes), so a bound of eight made every plan anew in each call
+// of five or more levels.  Five levels of 4 x 256 to 1024 x 4096 nodes: 3.8-18 ms a call with plans
+// made anew, 0.96 ms with plans kept (0.36 of it fbb_fill_kernel's Gaussians, 0.24 the transforms, 0.14
+// fbb_bridge_kernel, 0.36 before it shared the bridge's powers).  At most 32 are kept; the oldest is
+// dropped.
+constexpr size_t kFbbPlans = 32;
+
 static int fbb_plan(Ctx *c, int n2, int batch, cufftHandle *out)
 {
-    for (const auto &p : c->fbb_plans) {
-        if (p.n2 == n2 && p.batch == batch) {
-            *out = p.h;
-            return 0;
+    const Ctx::FftPlan *f = nullptr;
+    for (const auto &p : c->fbb_plans)
+        if (p.n2 == n2 && p.batch == batch) f = &p;
+    if (!f) {
+        if (c->fbb_plans.size() >= kFbbPlans) {
+            cufftDestroy(c->fbb_plans.front().h);
+            c->fbb_plans.erase(c->fbb_plans.begin());
         }
+        cufftHandle h = 0;
+        int n[1] = {n2};
+        size_t ws = 0;
+        FWT_CUFFT(cufftCreate(&h));
+        cufftResult r = cufftSetAutoAllocation(h, 0);
+        if (r == CUFFT_SUCCESS) r = cufftMakePlanMany(h, 1, n, nullptr, 1, n2, nullptr, 1, n2, CUFFT_Z2Z, batch, &ws);
+        if (r != CUFFT_SUCCESS) cufftDestroy(h);
+        FWT_CUFFT(r);
+        c->fbb_plans.push_back({n2, batch, h, ws});
+        f = &c->fbb_plans.back();
     }
-    if (c->fbb_plans.size() >= 8) {
-        cufftDestroy(c->fbb_plans.front().h);
-        c->fbb_plans.erase(c->fbb_plans.begin());
+    if (f->ws > c->fbb_ws_bytes) {
+        if (c->fbb_ws) cudaFree(c->fbb_ws);   // waits for the device
+        c->fbb_ws = nullptr;
+        c->fbb_ws_bytes = 0;
+        FWT_CUDA(cudaMalloc(&c->fbb_ws, f->ws));
+        c->fbb_ws_bytes = f->ws;
     }
-    cufftHandle h = 0;
-    int n[1] = {n2};
-    FWT_CUFFT(cufftPlanMany(&h, 1, n, nullptr, 1, n2, nullptr, 1, n2, CUFFT_Z2Z, batch));
-    c->fbb_plans.push_back({n2, batch, h});
-    *out = h;
+    FWT_CUFFT(cufftSetStream(f->h, c->stream));
+    if (f->ws) FWT_CUFFT(cufftSetWorkArea(f->h, c->fbb_ws));
+    *out = f->h;
     return 0;
 }
 
@@ -217,9 +241,8 @@ int fbb_generate(Ctx *c, uint64_t seed, int nlev, const int *tubes, const int *n
         fbb_row_kernel<<<(n2 + 255) / 256, 256, 0, c->stream>>>(M, H[lv], row);
         cufftHandle p1;
         FWT_TRY(fbb_plan(c, n2, 1, &p1));
-        FWT_CUFFT(cufftSetStream(p1, c->stream));
         FWT_CUFFT(cufftExecZ2Z(p1, row, row, CUFFT_FORWARD));
-        fbb_sqrt_kernel<<<(n2 + 255) / 256, 256, 0, c->stream>>>(n2, row, sq);
+        fbb_sqrt_kernel<<<(n2 + 255) / 256, 256, 0, c->stream>>>(n2, Np, H[lv], row, sq);
         c->launches += 3;
         // batches of tubes: 3 complex rows of n2 per tube, ~1 GB per batch
         const int per = std::max(1, (int)std::min<int64_t>(T, ((int64_t)1 << 30) / ((int64_t)3 * n2 * 16)));
@@ -233,10 +256,9 @@ int fbb_generate(Ctx *c, uint64_t seed, int nlev, const int *tubes, const int *n
             const int64_t tot = (int64_t)nb * n2;
             fbb_fill_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(seed, t0 + tb, nb, n2, sq, Zb);
             FWT_TRY(fbb_plan(c, n2, nb, &pb));
-            FWT_CUFFT(cufftSetStream(pb, c->stream));
             FWT_CUFFT(cufftExecZ2Z(pb, Zb, Zb, CUFFT_FORWARD));
             fbb_scan_kernel<<<nb, 256, 0, c->stream>>>(Zb, n2, M, fbm);
-            fbb_bridge_kernel<<<nt, 256, 0, c->stream>>>(seed, t0 + tb, Np, M, H[lv], dB[lv], fbm, d_x, d_y, d_z,
+            fbb_bridge_kernel<<<nt, 256, 0, c->stream>>>(seed, t0 + tb, Np, M, dB[lv], row, fbm, d_x, d_y, d_z,
                                                          node0 + (int64_t)tb * Np);
             c->launches += 4;
             FWT_CUDA(cudaGetLastError());
