@@ -325,22 +325,17 @@ __global__ void __launch_bounds__(kBuildThreads, 6) piece_build_kernel(
 }
 
 // ------------------------------------------------------------------------------ binning
-// Tiles of a piece: its box, culled to the tiles that meet at least one chord's box.
-template <typename F>
-__device__ __forceinline__ void for_each_tile(const PieceRec &S, int N, F &&f)
+// The binning's cull of a piece (box_tile): the tile meets at least one chord's box.
+__device__ __forceinline__ bool tile_cull(const PieceRec &S, int ox, int oy, int oz, int nx, int ny, int nz)
 {
     const int nch = S.nch;
-    for_each_box_tile(S.box_lo, S.box_hi, N,
-                      [&](int ox, int oy, int oz, int nx, int ny, int nz) {
-                          for (int j = 0; j < nch; ++j) {
-                              const uint32_t lo = __float_as_uint(S.chq[j].z), hi = __float_as_uint(S.chq[j].w);
-                              if (unpack3(lo, 0) <= ox + nx - 1 && unpack3(hi, 0) >= ox && unpack3(lo, 1) <= oy + ny - 1 &&
-                                  unpack3(hi, 1) >= oy && unpack3(lo, 2) <= oz + nz - 1 && unpack3(hi, 2) >= oz)
-                                  return true;
-                          }
-                          return false;
-                      },
-                      f);
+    for (int j = 0; j < nch; ++j) {
+        const uint32_t lo = __float_as_uint(S.chq[j].z), hi = __float_as_uint(S.chq[j].w);
+        if (unpack3(lo, 0) <= ox + nx - 1 && unpack3(hi, 0) >= ox && unpack3(lo, 1) <= oy + ny - 1 &&
+            unpack3(hi, 1) >= oy && unpack3(lo, 2) <= oz + nz - 1 && unpack3(hi, 2) >= oz)
+            return true;
+    }
+    return false;
 }
 
 // ------------------------------------------------------------------------------ deposit
@@ -1446,7 +1441,7 @@ int launch_piece(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
     int64_t *d_cnt = (int64_t *)C.scratch[20].p;
     int *d_err = (int *)(d_cnt + nrec + 1);
     FWT_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), c->stream));
-    const unsigned bq = (unsigned)((nrec + 255) / 256);
+    const unsigned bq = (unsigned)((nrec * kBinLanes + 255) / 256);
     int km = kt_begin(c, KT_BINNING);
     if (nrec > 0) pair_count_kernel<PieceRec><<<bq, 256, 0, c->stream>>>(B.piece, nrec, N, tz0, ntz, d_cnt, d_err);
     FWT_TRY(scan_exclusive_i64(c, d_cnt, nrec, d_cnt + nrec, C.scratch[12]));

@@ -55,15 +55,10 @@ __device__ __forceinline__ bool tile_may_hit(const SegRec &R, int ox, int oy, in
     return d2 <= __fmul_rn(rr, rr);
 }
 
-// Visit every (tile, image) of record S's box that may hold accepted points.
-template <typename F>
-__device__ __forceinline__ void for_each_tile(const SegRec &S, int N, F &&f)
+// The binning's cull of a record (box_tile).
+__device__ __forceinline__ bool tile_cull(const SegRec &S, int ox, int oy, int oz, int nx, int ny, int nz)
 {
-    for_each_box_tile(S.box_lo, S.box_hi, N,
-                      [&](int ox, int oy, int oz, int nx, int ny, int nz) {
-                          return tile_may_hit(S, ox, oy, oz, nx, ny, nz);
-                      },
-                      f);
+    return tile_may_hit(S, ox, oy, oz, nx, ny, nz);
 }
 
 // Counting sort, last step: every emitted pair to its tile's list.  Slots left unfilled by
@@ -815,7 +810,7 @@ int launch_tile(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
     int64_t *d_cnt = (int64_t *)C.scratch[20].p;
     int *d_err = (int *)(d_cnt + B.nsub + 1);
     FWT_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), c->stream));
-    const unsigned bq = (unsigned)((B.nsub + 255) / 256);
+    const unsigned bq = (unsigned)((B.nsub * kBinLanes + 255) / 256);
     int km = kt_begin(c, KT_BINNING);
     if (B.nsub > 0) pair_count_kernel<SegRec><<<bq, 256, 0, c->stream>>>(B.rec, B.nsub, N, tz0, ntz, d_cnt, d_err);
     FWT_TRY(scan_exclusive_i64(c, d_cnt, B.nsub, d_cnt + B.nsub, C.scratch[12]));
