@@ -82,6 +82,10 @@ __device__ __forceinline__ bool ref_tests_f64(const SubSeg &S, const double m[3]
     return rho < S.Rt;
 }
 
+// The vorticity of an accepted point.  General = false: a constant core and no twist, where the terms
+// along the normal and binormal are zero (eta and dsigma/ds are) and the value is tp Gamma T: 6 of 26
+// FP64 divisions and none of the frame.
+template <bool General>
 __device__ __forceinline__ void ref_value_f64(const SubSeg &S, const LineParam &P, const double *coe, double dtf,
                                               double dzeta_sup, double eta, const double m[3], double t0,
                                               double t1, double out[3])
@@ -89,15 +93,12 @@ __device__ __forceinline__ void ref_value_f64(const SubSeg &S, const LineParam &
     const double zeta = (S.s1 * t0 - S.s0 * t1) / S.ndci0;
     const double zsec = zeta - S.ssec;
     const double L = P.Len;
-    double cz[3], dc[3], ddc[3];
+    double cz[3], dc[3];
     spl_pos(coe, zsec * L, cz);
     const double dzeta = fmin(dzeta_sup, 1.0 * dtf);
     spl_d1(coe, zsec * L, dc);
     const double ndc = sqrt(dc[0] * dc[0] + dc[1] * dc[1] + dc[2] * dc[2]);
     double T[3] = {dc[0] / ndc, dc[1] / ndc, dc[2] / ndc};
-    spl_d2(coe, zsec * L, ddc);
-    double X[3] = {dc[1] * ddc[2] - dc[2] * ddc[1], dc[2] * ddc[0] - dc[0] * ddc[2], dc[0] * ddc[1] - dc[1] * ddc[0]};
-    const double nX = sqrt(X[0] * X[0] + X[1] * X[1] + X[2] * X[2]);
     double xc[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -113,6 +114,16 @@ __device__ __forceinline__ void ref_value_f64(const SubSeg &S, const LineParam &
     double tp = exp(-(rho * rho) / 2.0 / s2) / (dev_pi2() * s2);
     const double ftd = -exp(-(S.Rt * S.Rt) / 2.0 / s2) / (dev_pi2() * s2);
     tp = tp + ftd;
+    if constexpr (!General) {
+        // dsds = 0 and eta = 0: the terms along N and B below are zero
+#pragma unroll
+        for (int d = 0; d < 3; ++d) out[d] = tp * P.Gamma * T[d];
+        return;
+    }
+    double ddc[3];
+    spl_d2(coe, zsec * L, ddc);
+    double X[3] = {dc[1] * ddc[2] - dc[2] * ddc[1], dc[2] * ddc[0] - dc[0] * ddc[2], dc[0] * ddc[1] - dc[1] * ddc[0]};
+    const double nX = sqrt(X[0] * X[0] + X[1] * X[1] + X[2] * X[2]);
     const double sl = sigma_func(zeta - dzeta, P.length, P.sigma_max, P.sigma_min, P.n_T);
     const double sr = sigma_func(zeta + dzeta, P.length, P.sigma_max, P.sigma_min, P.n_T);
     double dsds = (sr - sl) / (2.0 * dzeta);
@@ -157,7 +168,7 @@ __device__ __forceinline__ bool point_ref_f64(const SubSeg &S, const LineParam &
     double m[3], t0, t1;
     ref_mesh_f64(dx, ip, jp, kp, m);
     if (!ref_tests_f64(S, m, t0, t1)) return false;
-    ref_value_f64(S, P, coe, dtf, dzeta_sup, eta, m, t0, t1, out);
+    ref_value_f64<true>(S, P, coe, dtf, dzeta_sup, eta, m, t0, t1, out);
     return true;
 }
 
@@ -293,7 +304,11 @@ __device__ __forceinline__ int redo_pair_f64(const RedoCtx &R, uint32_t rec, int
     ref_mesh_f64(dev_pi2() / R.N, ix[0], ix[1], ix[2], m);
     const bool pass = ref_tests_f64(S, m, t0, t1);
     if (decide && !pass) return 0;
-    ref_value_f64(S, P, R.coe + 18 * (size_t)slot, R.dtf[slot], R.dzeta_sup, R.eta, m, t0, t1, v);
+    const double *coe = R.coe + 18 * (size_t)slot;
+    if (P.sigma_max == P.sigma_min && R.eta == 0.0)
+        ref_value_f64<false>(S, P, coe, R.dtf[slot], R.dzeta_sup, R.eta, m, t0, t1, v);
+    else
+        ref_value_f64<true>(S, P, coe, R.dtf[slot], R.dzeta_sup, R.eta, m, t0, t1, v);
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {

@@ -725,7 +725,7 @@ __device__ __forceinline__ void drain_pieces(PieceStage &S, long long (*acc)[kAc
         redo_locate(redo, S.id[k] & ((1u << 26) - 1u), j, slot, jj);
         const int64_t q = redo.qoff[slot] + jj;
         const int *blo = redo.seg[q].box_lo;
-        ok64 = eval_pair_f64(redo, q, box_index(R.box_lo[0] + lx + B.dl[0], blo[0], redo.N),
+        ok64 = eval_pair_f64<General>(redo, q, box_index(R.box_lo[0] + lx + B.dl[0], blo[0], redo.N),
                       box_index(R.box_lo[1] + ly + B.dl[1], blo[1], redo.N),
                       box_index(R.box_lo[2] + lz + B.dl[2], blo[2], redo.N),
                       reinterpret_cast<double(*)[kAccN]>(acc), lx + kSY * ly + kSZ * lz);
@@ -823,13 +823,20 @@ template <bool General, bool Accumulate, bool F64, bool Raster>
 __global__ void __launch_bounds__(kDepThreads, F64 ? 2 : 3) deposit_piece_kernel(
     const PieceRec *__restrict__ rec, int N, int ntx, int nty, int tz0, const int64_t *__restrict__ tile_off,
     const uint32_t *__restrict__ list, double scale, void *__restrict__ wx, void *__restrict__ wy,
-    void *__restrict__ wz, int *__restrict__ err, const RedoCtx redo, const DeferList D,
-    const int64_t *__restrict__ ras_off, const uint32_t *__restrict__ ras_pts)
+    void *__restrict__ wz, int *__restrict__ err, const __grid_constant__ RedoCtx redo, const DeferList D,
+    const int64_t *__restrict__ ras_off, const uint32_t *__restrict__ ras_pts, int parts)
 {
     extern __shared__ __align__(16) unsigned char dsm[];
     long long(*acc)[kAccN] = reinterpret_cast<long long(*)[kAccN]>(dsm);
-    const int tile = (int)D.w0 + blockIdx.x;
-    const int64_t c0 = tile_off[tile], c1 = tile_off[tile + 1];
+    // an FP64 tile's records may be cut into parts (f64_parts)
+    const int tile = (int)D.w0 + (F64 ? (int)blockIdx.x / parts : (int)blockIdx.x);
+    const int part = F64 ? (int)blockIdx.x % parts : 0;
+    int64_t c0 = tile_off[tile], c1 = tile_off[tile + 1];
+    if (F64) {
+        const int64_t m = c1 - c0;
+        c1 = c0 + m * (part + 1) / parts;
+        c0 += m * part / parts;
+    }
     // a tile that no record of this batch meets keeps its values: earlier batches wrote them,
     // or the field was cleared before the first
     if (c0 == c1) return;
@@ -844,10 +851,13 @@ __global__ void __launch_bounds__(kDepThreads, F64 ? 2 : 3) deposit_piece_kernel
     // next one, so the warps of a tile end close together at the epilogue's barrier
     __shared__ int next_chunk;
     if (threadIdx.x == 0) next_chunk = kDepWarps;
-    if constexpr (F64)
-        tile_acc_init_f64<Accumulate>(reinterpret_cast<double(*)[kAccN]>(acc), N, x0, y0, z0, zs, zlim, (const double *)wx,
-                                      (const double *)wy, (const double *)wz);
-    else if (!D.emit_only)
+    if constexpr (F64) {
+        double(*a)[kAccN] = reinterpret_cast<double(*)[kAccN]>(acc);
+        if (parts > 1) tile_acc_init_f64<false>(a, N, x0, y0, z0, zs, zlim, nullptr, nullptr, nullptr);
+        else
+            tile_acc_init_f64<Accumulate>(a, N, x0, y0, z0, zs, zlim, (const double *)wx, (const double *)wy,
+                                          (const double *)wz);
+    } else if (!D.emit_only)
         tile_acc_init<Accumulate>(acc, N, x0, y0, z0, zs, zlim, scale, (const float *)wx, (const float *)wy,
                                   (const float *)wz);
     __syncthreads();
@@ -1005,10 +1015,11 @@ __global__ void __launch_bounds__(kDepThreads, F64 ? 2 : 3) deposit_piece_kernel
     if (failed && lane == 0) atomicOr(err, 2);
     if (lane == 0 && redo.tally && !D.emit_only) atomicAdd(redo.tally, (unsigned long long)nacc);
     __syncthreads();
-    if constexpr (F64)
-        tile_epilogue_f64(reinterpret_cast<double(*)[kAccN]>(acc), N, x0, y0, z0, zs, zlim, (double *)wx, (double *)wy,
-                          (double *)wz);
-    else if (!D.emit_only)
+    if constexpr (F64) {
+        double(*a)[kAccN] = reinterpret_cast<double(*)[kAccN]>(acc);
+        if (parts > 1) tile_add_f64(a, N, x0, y0, z0, zs, zlim, (double *)wx, (double *)wy, (double *)wz);
+        else tile_epilogue_f64(a, N, x0, y0, z0, zs, zlim, (double *)wx, (double *)wy, (double *)wz);
+    } else if (!D.emit_only)
         tile_epilogue(acc, N, x0, y0, z0, zs, zlim, scale, (float *)wx, (float *)wy, (float *)wz);
 }
 
@@ -1495,13 +1506,17 @@ int launch_piece(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
     rctx.tally = (unsigned long long *)((char *)C.scratch[19].p + 64);
     DeferList D{};
     if (!f64) FWT_TRY(defer_list(c, npairs, c->defer_per_pair, D));
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
+    const unsigned parts64 = f64 ? (unsigned)f64_parts(ntiles, sms) : 1u;
     auto launch = [&](const DeferList &L) -> int {
 #define FWT_PIECE_LAUNCH(G, A, F, R)                                                                       \
     do {                                                                                                   \
         FWT_CUDA(cudaFuncSetAttribute(deposit_piece_kernel<G, A, F, R>,                                    \
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPieceSmem));      \
-        deposit_piece_kernel<G, A, F, R><<<grid, kDepThreads, kPieceSmem, c->stream>>>(                   \
-            B.piece, N, ntx, nty, tz0, d_toff, d_list, scale, wx, wy, wz, d_err, rctx, L, B.ras_off, B.ras_pts); \
+        deposit_piece_kernel<G, A, F, R><<<grid * parts64, kDepThreads, kPieceSmem, c->stream>>>(                   \
+            B.piece, N, ntx, nty, tz0, d_toff, d_list, scale, wx, wy, wz, d_err, rctx, L, B.ras_off, B.ras_pts, \
+            (int)parts64);                                                                                 \
         FWT_CUDA(cudaGetLastError());                                                                      \
     } while (0)
 #define FWT_PIECE_LAUNCH_R(G, A, F)                                                                        \
@@ -1511,7 +1526,11 @@ int launch_piece(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
         const unsigned grid = (unsigned)(std::min<int64_t>(ntiles, L.w1) - L.w0);
         const int m = kt_begin(c, KT_DEPOSIT);
         if (f64) {
-            if (accumulate) FWT_PIECE_LAUNCH_R(true, true, true); else FWT_PIECE_LAUNCH_R(true, false, true);
+            if (general) {
+                if (accumulate) FWT_PIECE_LAUNCH_R(true, true, true); else FWT_PIECE_LAUNCH_R(true, false, true);
+            } else {
+                if (accumulate) FWT_PIECE_LAUNCH_R(false, true, true); else FWT_PIECE_LAUNCH_R(false, false, true);
+            }
         } else if (general) {
             if (accumulate) FWT_PIECE_LAUNCH_R(true, true, false); else FWT_PIECE_LAUNCH_R(true, false, false);
         } else {

@@ -229,7 +229,7 @@ __device__ __forceinline__ void drain_queue(WarpStage &S, long long (*acc)[kAccN
         lx = (int)((e >> 4) & 15u), ly = (int)((e >> 8) & 7u), lz = (int)((e >> 11) & 7u);
         const CandBox &B = S.box[k];
         const SegRec &R = S.rec[k];
-        ok64 = eval_pair_f64(redo, (int64_t)(S.id[k] & ((1u << 26) - 1u)), R.box_lo[0] + lx + B.dl[0],
+        ok64 = eval_pair_f64<General>(redo, (int64_t)(S.id[k] & ((1u << 26) - 1u)), R.box_lo[0] + lx + B.dl[0],
                       R.box_lo[1] + ly + B.dl[1], R.box_lo[2] + lz + B.dl[2], reinterpret_cast<double(*)[kAccN]>(acc),
                       lx + kSY * ly + kSZ * lz);
     } else if (lane < cnt) {
@@ -301,12 +301,19 @@ template <bool General, bool Accumulate, bool F64>
 __global__ void __launch_bounds__(kDepThreads, F64 ? 2 : 3) deposit_tile_kernel(
     const SegRec *__restrict__ rec, int N, int ntx, int nty, int tz0, const int64_t *__restrict__ tile_off,
     const uint32_t *__restrict__ list, double scale, void *__restrict__ wx, void *__restrict__ wy,
-    void *__restrict__ wz, int *__restrict__ err, const RedoCtx redo, const DeferList D)
+    void *__restrict__ wz, int *__restrict__ err, const __grid_constant__ RedoCtx redo, const DeferList D, int parts)
 {
     extern __shared__ __align__(16) unsigned char dsm[];
     long long(*acc)[kAccN] = reinterpret_cast<long long(*)[kAccN]>(dsm);
-    const int tile = (int)D.w0 + blockIdx.x;
-    const int64_t c0 = tile_off[tile], c1 = tile_off[tile + 1];
+    // an FP64 tile's records may be cut into parts (f64_parts)
+    const int tile = (int)D.w0 + (F64 ? (int)blockIdx.x / parts : (int)blockIdx.x);
+    const int part = F64 ? (int)blockIdx.x % parts : 0;
+    int64_t c0 = tile_off[tile], c1 = tile_off[tile + 1];
+    if (F64) {
+        const int64_t m = c1 - c0;
+        c1 = c0 + m * (part + 1) / parts;
+        c0 += m * part / parts;
+    }
     // a tile that no record of this batch meets keeps its values: earlier batches wrote them,
     // or the field was cleared before the first
     if (c0 == c1) return;
@@ -321,10 +328,13 @@ __global__ void __launch_bounds__(kDepThreads, F64 ? 2 : 3) deposit_tile_kernel(
     // next one, so the warps of a tile end close together at the epilogue's barrier
     __shared__ int next_rec;
     if (threadIdx.x == 0) next_rec = kDepWarps * kWarpChunk;
-    if constexpr (F64)
-        tile_acc_init_f64<Accumulate>(reinterpret_cast<double(*)[kAccN]>(acc), N, x0, y0, z0, zs, zlim, (const double *)wx,
-                                      (const double *)wy, (const double *)wz);
-    else if (!D.emit_only)
+    if constexpr (F64) {
+        double(*a)[kAccN] = reinterpret_cast<double(*)[kAccN]>(acc);
+        if (parts > 1) tile_acc_init_f64<false>(a, N, x0, y0, z0, zs, zlim, nullptr, nullptr, nullptr);
+        else
+            tile_acc_init_f64<Accumulate>(a, N, x0, y0, z0, zs, zlim, (const double *)wx, (const double *)wy,
+                                          (const double *)wz);
+    } else if (!D.emit_only)
         tile_acc_init<Accumulate>(acc, N, x0, y0, z0, zs, zlim, scale, (const float *)wx, (const float *)wy,
                                   (const float *)wz);
     __syncthreads();
@@ -450,10 +460,11 @@ __global__ void __launch_bounds__(kDepThreads, F64 ? 2 : 3) deposit_tile_kernel(
     if (failed && lane == 0) atomicOr(err, 2);
     if (lane == 0 && redo.tally && !D.emit_only) atomicAdd(redo.tally, (unsigned long long)nacc);
     __syncthreads();
-    if constexpr (F64)
-        tile_epilogue_f64(reinterpret_cast<double(*)[kAccN]>(acc), N, x0, y0, z0, zs, zlim, (double *)wx, (double *)wy,
-                          (double *)wz);
-    else if (!D.emit_only)
+    if constexpr (F64) {
+        double(*a)[kAccN] = reinterpret_cast<double(*)[kAccN]>(acc);
+        if (parts > 1) tile_add_f64(a, N, x0, y0, z0, zs, zlim, (double *)wx, (double *)wy, (double *)wz);
+        else tile_epilogue_f64(a, N, x0, y0, z0, zs, zlim, (double *)wx, (double *)wy, (double *)wz);
+    } else if (!D.emit_only)
         tile_epilogue(acc, N, x0, y0, z0, zs, zlim, scale, (float *)wx, (float *)wy, (float *)wz);
 }
 
@@ -866,14 +877,15 @@ int launch_tile(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
     const unsigned parts = (unsigned)block_parts(ntiles, sms, SegBlocks::kCtas);
+    const unsigned parts64 = f64 ? (unsigned)f64_parts(ntiles, sms) : 1u;
     const double dxg = kPi2 / N;   // as the records' dx
     auto launch = [&](const DeferList &L) -> int {
 #define FWT_TILE_LAUNCH(G, A, F)                                                                          \
     do {                                                                                                  \
         FWT_CUDA(cudaFuncSetAttribute(deposit_tile_kernel<G, A, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                       (int)kDepSmem));                                                    \
-        deposit_tile_kernel<G, A, F><<<grid, kDepThreads, kDepSmem, c->stream>>>(                         \
-            B.rec, N, ntx, nty, tz0, d_toff, d_list, scale, wx, wy, wz, d_err, rctx, L);                  \
+        deposit_tile_kernel<G, A, F><<<grid * parts64, kDepThreads, kDepSmem, c->stream>>>(                         \
+            B.rec, N, ntx, nty, tz0, d_toff, d_list, scale, wx, wy, wz, d_err, rctx, L, (int)parts64);     \
         FWT_CUDA(cudaGetLastError());                                                                     \
     } while (0)
         const unsigned grid = (unsigned)(std::min<int64_t>(ntiles, L.w1) - L.w0);
@@ -888,8 +900,11 @@ int launch_tile(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
         FWT_CUDA(cudaGetLastError());                                                                      \
     } while (0)
         if (f64) {
-            // the FP64 path evaluates every pair in FP64: the General distinction is only the FP32 one
-            if (accumulate) FWT_TILE_LAUNCH(true, true, true); else FWT_TILE_LAUNCH(true, false, true);
+            if (general) {
+                if (accumulate) FWT_TILE_LAUNCH(true, true, true); else FWT_TILE_LAUNCH(true, false, true);
+            } else {
+                if (accumulate) FWT_TILE_LAUNCH(false, true, true); else FWT_TILE_LAUNCH(false, false, true);
+            }
         } else if (general) {
             if (accumulate) FWT_TILE_LAUNCH(true, true, false); else FWT_TILE_LAUNCH(true, false, false);
         } else {

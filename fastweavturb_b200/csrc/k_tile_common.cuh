@@ -4,6 +4,8 @@
 // accumulator (set-up and the coalesced epilogue).
 #pragma once
 
+#include <algorithm>
+
 #include "k_deposit.cuh"
 
 namespace fwt {
@@ -313,11 +315,42 @@ __device__ __forceinline__ void tile_epilogue_f64(double (*acc)[kAccN], int N, i
     }
 }
 
+// The FP64 sums of one part of a tile's records, added into the field (cleared before the first batch).
+__device__ __forceinline__ void tile_add_f64(double (*acc)[kAccN], int N, int x0, int y0, int z0, int zs, int zlim,
+                                             double *__restrict__ wx, double *__restrict__ wy, double *__restrict__ wz)
+{
+    for (int p = threadIdx.x; p < TP; p += blockDim.x) {
+        const int lx = p % TX, ly = (p / TX) % TY, lz = p / (TX * TY);
+        const int gx = x0 + lx, gy = y0 + ly, gz = z0 + lz;
+        if (gx >= N || gy >= N || gz >= zlim) continue;
+        const size_t g = (size_t)gx + (size_t)N * ((size_t)gy + (size_t)N * (gz - zs));
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double v = acc[d][lx + kSY * ly + kSZ * lz];
+            double *w = d == 0 ? wx : (d == 1 ? wy : wz);
+            if (v != 0.0) atomicAdd(w + g, v);
+        }
+    }
+}
+
+// Parts that an FP64 tile's records are cut into, each with its own CTA and sums: enough for eight
+// waves of two CTAs per SM, at most eight.  A pair takes microseconds of dependent FP64 arithmetic, and
+// the 256 tiles of 64^3 left 40 of 148 SMs with one CTA and all of them waiting for the fullest tile.
+// Pieces and sub-segments of 64^3 (17 M pairs, ms): one part 7.8 and 1.9, with the constant core's
+// shorter evaluation (ref_value_f64) in 4 parts 3.7 and 0.8, with eval_pair_f64 called instead of
+// inlined 2.7 and 0.8, in 8 parts 2.5 and 0.8, in 9 the same.
+inline int f64_parts(int64_t ntiles, int sms)
+{
+    return (int)std::max<int64_t>(1, std::min<int64_t>(8, (int64_t)sms * 16 / std::max<int64_t>(ntiles, 1)));
+}
+
 // The FP64 tile path's evaluation of a candidate pair: the reference's FP64 tests of
 // tube.f90:806-818 at the 1-based unwrapped grid index (ip, jp, kp) of sub-segment q's own box,
 // and, if it passes, the reference's FP64 vorticity (tube.f90:819-892) added into the double
-// cell p.
-__device__ __forceinline__ bool eval_pair_f64(const RedoCtx &R, int64_t q, int ip, int jp, int kp,
+// cell p.  A call: inlined at each of the kernels' queue drains, the divisions and exponentials
+// overran the instruction cache (half of all stalls).
+template <bool General>
+__device__ __noinline__ bool eval_pair_f64(const RedoCtx &R, int64_t q, int ip, int jp, int kp,
                                               double (*acc)[kAccN], int p)
 {
     const SubSeg &S = R.seg[q];
@@ -325,9 +358,9 @@ __device__ __forceinline__ bool eval_pair_f64(const RedoCtx &R, int64_t q, int i
     ref_mesh_f64(dev_pi2() / R.N, ip, jp, kp, m);
     if (!ref_tests_f64(S, m, t0, t1)) return false;
     const int slot = S.slot;
-    const LineParam P = R.lp[R.slot_line[slot]];
+    const LineParam &P = R.lp[R.slot_line[slot]];
     double v[3];
-    ref_value_f64(S, P, R.coe + 18 * (size_t)slot, R.dtf[slot], R.dzeta_sup, R.eta, m, t0, t1, v);
+    ref_value_f64<General>(S, P, R.coe + 18 * (size_t)slot, R.dtf[slot], R.dzeta_sup, R.eta, m, t0, t1, v);
 #pragma unroll
     for (int d = 0; d < 3; ++d) atomicAdd(&acc[d][p], v[d]);
     return true;
