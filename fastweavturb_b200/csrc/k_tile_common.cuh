@@ -68,6 +68,16 @@ __device__ __forceinline__ bool box_tile(const Rec &S, const BoxTiles &B, int N,
     return tile_cull(S, o[0], o[1], o[2], n[0], n[1], n[2]);
 }
 
+// warp-aggregated increment of cnt[key]
+__device__ __forceinline__ void agg_inc(uint32_t *cnt, uint32_t key, bool active)
+{
+    const unsigned act = __ballot_sync(0xffffffffu, active);
+    if (!active) return;
+    const unsigned peers = __match_any_sync(act, key);
+    const int leader = __ffs(peers) - 1;
+    if ((int)(threadIdx.x & 31) == leader) atomicAdd(cnt + key, (uint32_t)__popc(peers));
+}
+
 constexpr uint32_t kNoTile = 0xffffffffu;   // key of a pair slot that the emitting pass left empty
 
 // Binning, step 1: number of (tile, image) pairs of every record, in the tiles of the context's z-slab
@@ -77,6 +87,8 @@ constexpr uint32_t kNoTile = 0xffffffffu;   // key of a pair slot that the emitt
 // record the warp waited for its largest and wrote its pairs to 32 places.  Bound by the culls' issue
 // and by the pairs' writes; both steps for the records of 73 lines of 148 nodes (200^3, cores varying by
 // four), one thread a record -> eight lanes: sub-segments 0.58 -> 0.05 ms, pieces 0.32 -> 0.05 ms.
+// The tiles' counts are added up within the warp first: the 256 counters of 64^3 took 0.17 ms for 1 M
+// pairs one by one, 0.08 ms so.
 constexpr int kBinLanes = 8;
 
 template <typename Rec>
@@ -136,12 +148,13 @@ __global__ void pair_emit_kernel(const Rec *__restrict__ seg, int64_t nsub, int 
         // the record's lanes take consecutive slots, in the order of the tiles
         const unsigned bal = (__ballot_sync(0xffffffffu, hit) >> (lane - sub)) & ((1u << kBinLanes) - 1u);
         const int64_t s = o + __popc(bal & ((1u << sub) - 1u));
-        if (hit && s < end) {
-            const uint32_t tile = (uint32_t)(t[0] + ntx * (t[1] + nty * (t[2] - tz0)));
+        const uint32_t tile = (uint32_t)(t[0] + ntx * (t[1] + nty * (t[2] - tz0)));
+        const bool put = hit && s < end;
+        if (put) {
             key[s] = tile;
             val[s] = (uint32_t)q | (img << 26);
-            atomicAdd(tile_cnt + tile, 1u);
         }
+        agg_inc(tile_cnt, tile, put);   // neighbouring records meet the same tiles
         o += __popc(bal);
     }
     for (o += sub; o < end; o += kBinLanes) key[o] = kNoTile;
