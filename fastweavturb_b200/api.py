@@ -367,7 +367,7 @@ class Context:
 
     def set_scatter_radius_limit(self, cells):
         """FP32 piece tubes up to this truncation radius (grid spacings) are deposited without
-        tiles, with int64 global reductions (0: never; negative: the default, 5, or 8 with a constant core)."""
+        tiles, with int64 global reductions (0: never; negative: the default, 8)."""
         _check(library().fwt_set_tuning(self._h, 3, float(cells)))
 
     def set_defer_limit(self, pairs):

@@ -168,7 +168,6 @@ int deposit_lines(Ctx *c, int line_s, int line_e)
     // radius limit of the piece kernel in grid spacings: fwt_set_tuning, else the environment
     // variable FWT_PIECE_RT_CELLS, else the default
     const char *env = std::getenv("FWT_PIECE_RT_CELLS");
-    const bool const32 = c->p.precision == 32 && c->p.sigma_ratio == 1.0 && c->p.eta_t == 0.0;
     const double rt_cells = c->piece_rt_cells >= 0.0 ? c->piece_rt_cells : (env ? std::atof(env) : kPieceMaxRtCells);
     auto thin = [&](int l) {
         return tile_path && c->p.Rtube_ratio * c->p.sigma_ratio * c->sigma[l] <= rt_cells * dxg;
@@ -185,7 +184,7 @@ int deposit_lines(Ctx *c, int line_s, int line_e)
     const char *senv = std::getenv("FWT_SCATTER_RT_CELLS");
     const double sca_cells =
         c->scatter_rt_cells >= 0.0 ? c->scatter_rt_cells
-                                   : (senv ? std::atof(senv) : (const32 ? kScatterMaxRtCellsConst : kScatterMaxRtCells));
+                                   : (senv ? std::atof(senv) : kScatterMaxRtCells);
     auto scattered = [&](int l) {
         return thin(l) && c->p.precision == 32 && !rasterised(l) &&
                c->p.Rtube_ratio * c->p.sigma_ratio * c->sigma[l] <= sca_cells * dxg;

@@ -765,13 +765,10 @@ constexpr double kPieceMaxRtCells = 8.0;
 constexpr double kRasterMaxRtCells = 0.0;
 // Piece lines whose truncation radius is at most this many grid spacings are deposited without
 // tiles (scatter_piece_kernel, FP32 only): each piece is searched once and its contributions
-// added with int64 global reductions, instead of once in every tile its box meets.  On the
-// 1024^3 workload the scatter path took 0.34x (radius 1.9 grid spacings) and 0.75x (3.8) of the
-// tile path's deposition time, and 1.5x at 7.6, where a chord accepts hundreds of points.
-constexpr double kScatterMaxRtCells = 5.0;
-// With a constant core the tile-free path is the faster one up to the piece limit (512^3, 512
-// tubes of 4096 nodes, ms against the piece tile kernel: 5.5: 114 / 135, 6.5: 189 / 205, 7.6:
-// 308 / 306).
-constexpr double kScatterMaxRtCellsConst = 8.0;
+// added with int64 global reductions, instead of once in every tile its box meets.  It is the faster
+// path up to the piece limit.  Constant cores (512^3, 512 tubes of 4096 nodes, ms against the piece
+// tile kernel): 5.5: 76 / 135, 7.6: 204 / 306.  Cores varying by four (200^3, 73 lines of 148 nodes,
+// a whole field): 4.9 with all its piece lines without tiles, 5.4 with those above 5 in tiles.
+constexpr double kScatterMaxRtCells = 8.0;
 
 }  // namespace fwt
