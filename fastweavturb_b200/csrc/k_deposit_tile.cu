@@ -327,7 +327,8 @@ __global__ void __launch_bounds__(kDepThreads, F64 ? 2 : 3) deposit_tile_kernel(
     // chunks are handed out through a shared counter: a warp that finishes early takes the
     // next one, so the warps of a tile end close together at the epilogue's barrier
     __shared__ int next_rec;
-    if (threadIdx.x == 0) next_rec = kDepWarps * kWarpChunk;
+    const int first = max(1, min(kWarpChunk, (int)((c1 - c0) / (2 * kDepWarps))));   // candidates in a warp's first chunk
+    if (threadIdx.x == 0) next_rec = kDepWarps * first;
     if constexpr (F64) {
         double(*a)[kAccN] = reinterpret_cast<double(*)[kAccN]>(acc);
         if (parts > 1) tile_acc_init_f64<false>(a, N, x0, y0, z0, zs, zlim, nullptr, nullptr, nullptr);
@@ -346,8 +347,8 @@ __global__ void __launch_bounds__(kDepThreads, F64 ? 2 : 3) deposit_tile_kernel(
     bool failed = false;
     int qn = 0;   // queued points of this warp (warp-uniform)
     unsigned nacc = 0;   // pairs evaluated by this warp (warp-uniform)
-    int csz = kWarpChunk;   // candidates in this warp's current chunk
-    for (int start = warp * kWarpChunk; start < nrec && !failed;) {
+    int csz = first;   // candidates in this warp's current chunk
+    for (int start = warp * first; start < nrec && !failed;) {
         const int64_t base = c0 + start;
         const int nc = min(csz, nrec - start);
         const uint32_t v = lane < nc ? __ldg(list + base + lane) : 0u;
@@ -446,12 +447,12 @@ __global__ void __launch_bounds__(kDepThreads, F64 ? 2 : 3) deposit_tile_kernel(
         if (qn > 0) drain_queue<General, F64>(S, acc, lane, qn, qn, nacc, fscale, fmaxq, err, redo, D, x0, y0, z0);
         __syncwarp();   // the warp's stage is reused by its next chunk
         // the next chunk, guided self-scheduling: kWarpChunk candidates while many remain,
-        // down to two near the end of the list, so that the warps reach the epilogue's
+        // down to one near the end of the list, so that the warps reach the epilogue's
         // barrier close together (a thick tube's candidates cost a whole tile each)
         int nxt = 0, cs = 0;
         if (lane == 0) {
             const int rem = nrec - *(volatile int *)&next_rec;
-            cs = max(2, min(kWarpChunk, rem / (2 * kDepWarps)));
+            cs = max(1, min(kWarpChunk, rem / (2 * kDepWarps)));
             nxt = atomicAdd(&next_rec, cs);
         }
         start = __shfl_sync(0xffffffffu, nxt, 0);
