@@ -6,18 +6,20 @@
 // 2. counting sort by tile: integer histogram, exclusive scan, scatter (warp-aggregated
 //    atomics) -> per-tile candidate lists holding exactly the sub-segments whose box meets
 //    the tile.
-// 3. deposit_tile_kernel: one CTA per tile, accumulating the tile in shared int64 fixed-point
-//    cells.  Integer addition is associative, so the tile sum is bit-exact whatever the order
-//    of candidates.  Each warp claims chunks of candidates and stages their FP32 records with
-//    one bulk asynchronous copy each (cp.async.bulk, the TMA engine's 1-D form, completing on
-//    the warp's mbarrier).  A chunk's work is flattened into grid rows along each candidate's
-//    best-aligned axis; each row solves the two half-space tests and the cylinder test of
-//    tube.f90:806-818 for its index interval (one-point margin) and evaluates the reference
-//    predicate and vorticity only there, where the reference walks the whole box (about 11
-//    points per accepted one at these sub-segment lengths).  A point whose plane test lies
-//    within its FP32 rounding bound of zero is decided by the reference's FP64 tests, and
-//    evaluated in FP64 if accepted: the field jumps across the plane two consecutive chords
-//    share.  The tile is written once with coalesced float4 stores.
+// 3. one CTA per tile accumulates the tile in int64 fixed-point cells, whose sums do not depend on
+//    the order of the candidates:
+//    - FP32 lines with a constant core: deposit_block_kernel (k_block.cuh) with the SegBlocks policy
+//      below, every point of a 4 x 4 x 4 block against each record that may reach it;
+//    - varying cores, and the FP64 path (double cells): deposit_tile_kernel.  Each warp claims chunks
+//      of candidates and stages their FP32 records with one bulk asynchronous copy each
+//      (cp.async.bulk, completing on the warp's mbarrier).  A chunk's work is flattened into grid
+//      rows along each candidate's best-aligned axis; each row solves the two half-space tests
+//      and the cylinder test of tube.f90:806-818 for its index interval (one-point margin) and
+//      tests and evaluates the points only there.
+//    A point whose plane test lies within its FP32 rounding bound of zero is decided by the
+//    reference's FP64 tests, and evaluated in FP64 if accepted: the field jumps across the plane
+//    two consecutive chords share.  The tile is written once, with 16-byte stores where the rows
+//    of omega allow it.
 #include <cstdio>
 #include <cstdlib>
 
