@@ -148,6 +148,22 @@ constexpr int kMlpBN = 32, kMlpStages = 4, kMlpThreads = 256;
 constexpr size_t kMlpStage = (size_t)(kGemmBM + kMlpBN) * kGemmBK * 2;
 constexpr size_t kMlpSmem = kMlpStage * kMlpStages;
 
+// The ring's copies: cp.async group c holds chunk c.  The prologue commits groups 0 .. kMlpStages - 1;
+// iteration kc >= 1 refills the stage of chunk kc - 1 and commits group kc - 1 + kMlpStages (empty past the
+// last chunk), iteration 0 commits none.  Groups that may still be in flight when iteration kc issues its
+// products, so that groups 0 .. kc have landed:
+constexpr int ring_pending(int kc) { return kc == 0 ? kMlpStages - 1 : kMlpStages - 2; }
+constexpr bool ring_covers(int nk)
+{
+    int committed = kMlpStages;
+    for (int kc = 0; kc < nk; ++kc) {
+        if (committed - ring_pending(kc) < kc + 1) return false;
+        if (kc > 0 && committed++ != kc - 1 + kMlpStages) return false;   // group c is chunk c
+    }
+    return true;
+}
+static_assert(ring_covers(4096), "mlp_gemm_kernel: a chunk is multiplied before its copies have landed");
+
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool in)
 {
     const int n = in ? 16 : 0;   // rows beyond the matrix read zeros
@@ -252,7 +268,8 @@ __global__ void __launch_bounds__(kMlpThreads) mlp_gemm_kernel(const __grid_cons
     }
     bool ok = true;
     for (int kc = 0; kc < nk && ok; ++kc) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kMlpStages - 1) : "memory");
+        if (kc == 0) asm volatile("cp.async.wait_group %0;" ::"n"(ring_pending(0)) : "memory");
+        else asm volatile("cp.async.wait_group %0;" ::"n"(ring_pending(1)) : "memory");
         // the MMA reads shared memory through the async proxy
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
@@ -284,7 +301,7 @@ __global__ void __launch_bounds__(kMlpThreads) mlp_gemm_kernel(const __grid_cons
                 load_a(nx);
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (kc > 0) asm volatile("cp.async.commit_group;" ::: "memory");
     }
     if (ok) {
         ok = gemm_mbar_wait(bar0 + 8u * (uint32_t)((nk - 1) % kMlpStages), (uint32_t)((nk - 1) / kMlpStages) & 1u);
