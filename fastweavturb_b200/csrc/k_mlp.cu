@@ -61,8 +61,9 @@ struct fwt_mlp {
     std::vector<fwt::MlpLayer> L;
     __nv_bfloat16 *X0 = nullptr, *X0t = nullptr;   // B x 64, 64 x B
     // One exchange buffer with the host, and its mirror there: the loss (FP64), the error flag and a
-    // pad, then x (B x n_in; the input gradient replaces it), then the targets (B x n_out; the
-    // forward pass writes its outputs there), then the output weights (n_out).
+    // pad, then x (B x n_in; the input gradient replaces it), then from the next 16 bytes on the targets
+    // (B x n_out; the forward pass writes its outputs there, 16 bytes a store), then the output weights
+    // (n_out).
     // The mirror is ordinary memory: pinning it cost 14-25 ms a network and saved nothing measurable a step.
     unsigned char *io = nullptr;
     std::vector<unsigned char> hmem;
@@ -73,7 +74,8 @@ struct fwt_mlp {
 
     int *err() const { return (int *)(io + 8); }
     float *x() const { return (float *)(io + 16); }
-    float *t(int B) const { return x() + (size_t)B * n_in; }
+    size_t t_at(int B) const { return ((size_t)B * n_in + 3) / 4 * 4; }   // floats from x to the targets
+    float *t(int B) const { return x() + t_at(B); }
     float *w(int B) const { return t(B) + (size_t)B * n_out; }
 };
 
@@ -239,7 +241,7 @@ __global__ void __launch_bounds__(kMlpThreads) mlp_gemm_kernel(const __grid_cons
     const bool in_b = row < (J.epi == kWeight ? J.M : J.B);
     const int nc = in_b ? max(0, min(16, J.Nl - c0)) : 0;   // this thread's columns inside the result
     const size_t at = (size_t)row * J.Nl + c0;
-    const bool vec = nc == 16 && (J.Nl & 3) == 0;           // its 16 values start on 16 bytes
+    const bool vec = nc == 16 && (J.Nl & 3) == 0;           // its 16 values start on 16 bytes, as every result does
     float e0[16], e1[16], e2[16];   // bias or Z; targets; output weights
 #pragma unroll
     for (int i = 0; i < 16; ++i) e0[i] = e1[i] = e2[i] = 0.0f;
@@ -633,6 +635,7 @@ static int mlp_upload(fwt_mlp *m, const float *x, const float *t, const float *w
     std::memcpy(h, x, sizeof(float) * (size_t)B * m->n_in);
     size_t n = (size_t)B * m->n_in;
     if (t) {
+        n = m->t_at(B);
         std::memcpy(h + n, t, sizeof(float) * (size_t)B * m->n_out);
         n += (size_t)B * m->n_out;
         for (int i = 0; i < m->n_out; ++i) h[n + i] = w_out ? w_out[i] : 1.0f;
@@ -739,6 +742,7 @@ int fwt_mlp_create(int device, int n_in, int width, int depth, int n_out, int ba
     }
     try_(mlp_alloc(m, &m->X0, (size_t)Bp * 64));
     try_(mlp_alloc(m, &m->X0t, (size_t)64 * Bp));
+    // (Bp x n_in is a multiple of four floats: no batch needs more)
     const size_t io_bytes = kIoHead + sizeof(float) * ((size_t)Bp * (n_in + n_out) + n_out);
     try_(mlp_alloc(m, &m->io, io_bytes));
     m->hmem.resize(io_bytes);
@@ -812,7 +816,7 @@ int fwt_mlp_forward(fwt_mlp *m, const float *x, int batch, float *y)
     cudaSetDevice(m->dev);
     FWT_TRY(mlp_upload(m, x, nullptr, nullptr, batch));
     FWT_TRY(mlp_forward(m, batch, false));
-    const size_t nx = (size_t)batch * m->n_in, ny = (size_t)batch * m->n_out;
+    const size_t nx = m->t_at(batch), ny = (size_t)batch * m->n_out;
     FWT_TRY(mlp_download(m, nx + ny));
     std::memcpy(y, m->hio + kIoHead + sizeof(float) * nx, sizeof(float) * ny);
     return 0;
