@@ -24,6 +24,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <string>
 #include <vector>
 
@@ -745,8 +746,14 @@ int fwt_mlp_create(int device, int n_in, int width, int depth, int n_out, int ba
     // (Bp x n_in is a multiple of four floats: no batch needs more)
     const size_t io_bytes = kIoHead + sizeof(float) * ((size_t)Bp * (n_in + n_out) + n_out);
     try_(mlp_alloc(m, &m->io, io_bytes));
-    m->hmem.resize(io_bytes);
-    m->hio = m->hmem.data();
+    if (rc == 0) {   // a failed device allocation leaves no reason to ask the host for as much
+        try {
+            m->hmem.resize(io_bytes);
+        } catch (const std::exception &) {
+            rc = fail(FWT_E_NOMEM, "mlp: host allocation failed");
+        }
+        m->hio = m->hmem.data();
+    }
     if (rc == 0 && cudaFuncSetAttribute(mlp_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMlpSmem) != cudaSuccess)
         rc = fail(FWT_E_CUDA, "mlp: kernel attribute");
     if (rc == 0) rc = mlp_refresh_all(m);
