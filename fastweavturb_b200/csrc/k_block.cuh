@@ -136,6 +136,9 @@ __global__ void __launch_bounds__(kDepThreads, Policy::kCtas) deposit_block_kern
         acc[1][pa] = a1;
         acc[2][pa] = a2;
     }
+    // the first chunk's record ids, written by warp 0 with plain stores, are read by every warp (the
+    // barriers of the chunk loop order the later ones; the mbarrier orders the bulk copies alone)
+    __syncthreads();
 
     // an emit-only pass lists the deferred pairs again and discards its sums
     const float fscale = D.emit_only ? 0.0f : (float)scale;
