@@ -135,9 +135,9 @@ __global__ void __launch_bounds__(256) pdf_kernel(const Real *__restrict__ a, si
 // Bound by FP64 arithmetic: the sums of du^p, p = 1..PMAX, over every point and separation.  A
 // warp takes MPW separations and a share of the positions, so a point is read and widened once
 // for MPW increments; the sums use the even powers and fused multiply-adds (8 FP64 operations
-// for p <= 6, 14 for 10, where a running power took 21), the scale 1/u' enters as an exact power
-// of two when the lines are staged and as its remainder at the end, only as many orders as
-// asked for are summed, and separations equal modulo N once (the host's list).  512^3, three
+// for p <= 6, 14 for 10, where a running power took 21), the scale s = 1/u' enters as the power of
+// two just above it, exactly, when the lines are staged, and as the remainder in [0.5, 1) at the end,
+// only as many orders as asked for are summed, and separations equal modulo N once (the host's list).  512^3, three
 // components, orders 1-6: 14.5 ms with the running power to order 10, 7.8 now; at the FP64 rate
 // the 17 separations take 3.8.
 template <typename Real>
@@ -178,11 +178,13 @@ __device__ __forceinline__ void sp_accumulate(double d, double (&acc)[PMAX])
 // the whole grid, or a z-slab (axes 0, 1) or y-pencil (axis 2) of a grid split over GPUs.  The
 // axis is axis0 + blockIdx.y, its component stride elements further on per step.  blockDim is
 // 32 x (groups of separations) x (1 or 2 shares of the positions).
-// Groups beyond eight go to blockIdx.z.
-template <typename Real, int PMAX>
+// Groups beyond eight go to blockIdx.z.  Scaled: each increment is multiplied by `post` in FP64, for a
+// scale that says nothing about the field's size (a caller's own, or one beyond the staged type's
+// exponents), where sc is 1.
+template <typename Real, int PMAX, bool Scaled = false>
 __global__ void __launch_bounds__(kSpMaxThreads, PMAX > 6 ? 1 : 2) sp_kernel(const Real *__restrict__ u0, size_t stride, int N, int n0, int n1, int n2,
-                                                 int axis0, Real sc, const int *__restrict__ rs, int nr,
-                                                 double *__restrict__ Sp)
+                                                 int axis0, Real sc, double post, const int *__restrict__ rs,
+                                                 int nr, double *__restrict__ Sp)
 {
     extern __shared__ __align__(16) unsigned char sp_smem[];
     Real *tile = reinterpret_cast<Real *>(sp_smem);   // N x (W + 1)
@@ -236,7 +238,8 @@ __global__ void __launch_bounds__(kSpMaxThreads, PMAX > 6 ? 1 : 2) sp_kernel(con
                 for (int a = 0; a < kSpPerWarp; ++a) {
                     int q = pos + rr[a];
                     if (q >= N) q -= N;
-                    sp_accumulate<PMAX>((double)tile[q * ld + line] - c, acc[a]);
+                    const double d = (double)tile[q * ld + line] - c;
+                    sp_accumulate<PMAX>(Scaled ? d * post : d, acc[a]);
                 }
             }
         }
@@ -425,9 +428,10 @@ int stats_pdf(Ctx *c, int which, int comp, int nbins, float *val, float *pdf, ui
 
 // Sums of du^p, p = 1..pmax, on a box (n0 x n1 x n2) of `axes` consecutive axes from axis0 (one
 // component each, `stride` elements apart): sums[(p - 1) * nr + m] = sum (du s)^p at separation
-// r[m].  Separations equal modulo N are summed once.
-static int sp_sums(Ctx *c, const void *u, size_t stride, int n0, int n1, int n2, int axis0, int axes, double s, int pmax,
-                   const int *r, int nr, double *sums)
+// r[m].  Separations equal modulo N are summed once.  own_scale: s is 1/u' of this very field, so that
+// u s is of order one.
+static int sp_sums(Ctx *c, const void *u, size_t stride, int n0, int n1, int n2, int axis0, int axes, double s,
+                   bool own_scale, int pmax, const int *r, int nr, double *sums)
 {
     const int N = c->p.N;
     const bool f64 = c->p.precision == 64;
@@ -447,12 +451,17 @@ static int sp_sums(Ctx *c, const void *u, size_t stride, int n0, int n1, int n2,
         if (i == uniq.size()) uniq.push_back(q);
         at[m] = (int)i;
     }
-    const int P = pmax <= 4 ? 4 : (pmax <= 6 ? 6 : 10), nu = (int)uniq.size();
-    std::vector<double> h((size_t)P * nu);
-    // the power of two nearest 1 / s scales the staged lines exactly; the rest is applied below
+    // the power of two just above s scales the staged lines exactly; the rest, in [0.5, 1), is applied
+    // below.  Any other scale (zero, negative, not finite, or beyond the staged type's exponents) and a
+    // scale that need not fit the field, whose product with it could leave that type's range, multiplies
+    // each increment in FP64 instead
     int e = 0;
     std::frexp(s, &e);
-    const double sc = std::isfinite(s) && s > 0 && e > -100 && e < 100 ? std::ldexp(1.0, e) : 1.0;
+    const int emax = f64 ? 1000 : 120;
+    const bool staged = own_scale && std::isfinite(s) && s > 0 && e > -emax && e < emax;
+    const double sc = staged ? std::ldexp(1.0, e) : 1.0;
+    const int P = !staged ? 10 : (pmax <= 4 ? 4 : (pmax <= 6 ? 6 : 10)), nu = (int)uniq.size();
+    std::vector<double> h((size_t)P * nu);
     FWT_TRY(buf_reserve(c, c->scratch[9], sizeof(int) * 64 + sizeof(double) * 10 * 64 + 64));
     int *d_r = (int *)c->scratch[9].p;
     double *d_sp = (double *)((char *)c->scratch[9].p + 256);
@@ -466,16 +475,18 @@ static int sp_sums(Ctx *c, const void *u, size_t stride, int n0, int n1, int n2,
     const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)sms * 2)), (unsigned)axes,
                     (unsigned)((all + kSpGroups - 1) / kSpGroups));
     const int km = kt_begin(c, KT_STATS);
-#define FWT_SP(REAL, PM)                                                                                           \
+#define FWT_SP(REAL, ...)                                                                                          \
 do {                                                                                                           \
-    auto k = sp_kernel<REAL, PM>;                                                                              \
+    auto k = sp_kernel<REAL, __VA_ARGS__>;                                                                     \
     FWT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));                    \
-    k<<<grid, threads, shb, c->stream>>>((const REAL *)u, stride, N, n0, n1, n2, axis0, (REAL)sc, d_r, nu, d_sp); \
+    k<<<grid, threads, shb, c->stream>>>((const REAL *)u, stride, N, n0, n1, n2, axis0, (REAL)sc, s, d_r, nu, d_sp); \
 } while (0)
     if (f64) {
-        if (P == 4) FWT_SP(double, 4); else if (P == 6) FWT_SP(double, 6); else FWT_SP(double, 10);
+        if (!staged) FWT_SP(double, 10, true); else if (P == 4) FWT_SP(double, 4);
+        else if (P == 6) FWT_SP(double, 6); else FWT_SP(double, 10);
     } else {
-        if (P == 4) FWT_SP(float, 4); else if (P == 6) FWT_SP(float, 6); else FWT_SP(float, 10);
+        if (!staged) FWT_SP(float, 10, true); else if (P == 4) FWT_SP(float, 4);
+        else if (P == 6) FWT_SP(float, 6); else FWT_SP(float, 10);
     }
 #undef FWT_SP
     kt_end(c, km);
@@ -485,7 +496,7 @@ do {                                                                            
     FWT_CUDA(cudaStreamSynchronize(c->stream));
     double f = 1.0;
     for (int p = 0; p < pmax; ++p) {
-        f *= s / sc;
+        f *= staged ? s / sc : 1.0;
         for (int m = 0; m < nr; ++m) sums[p * nr + m] = h[(size_t)p * nu + at[m]] * f;
     }
     return 0;
@@ -500,7 +511,7 @@ int stats_sp(Ctx *c, int pmax, const int *r, int nr, double *Sp)
     const int N = c->p.N;
     for (int m = 0; m < nr; ++m)
         if (r[m] < 0) return fail(FWT_E_ARG, "Sp: negative separation");
-    FWT_TRY(sp_sums(c, c->b_u.p, field_elems(c), N, N, N, 0, 3, 1.0 / c->up, pmax, r, nr, Sp));
+    FWT_TRY(sp_sums(c, c->b_u.p, field_elems(c), N, N, N, 0, 3, 1.0 / c->up, true, pmax, r, nr, Sp));
     const double inv = 1.0 / ((double)N * N * N * 3.0);
     for (int i = 0; i < pmax * nr; ++i) Sp[i] *= inv;
     return 0;
@@ -573,7 +584,7 @@ int stats_sp_block(Ctx *c, const void *u, int n0, int n1, int n2, int axis, doub
     if (nr < 1 || nr > 64) return fail(FWT_E_ARG, "sp_block: nr must be 1..64");
     for (int m = 0; m < nr; ++m)
         if (r[m] < 0) return fail(FWT_E_ARG, "sp_block: negative separation");
-    return sp_sums(c, u, 0, n0, n1, n2, axis, 1, s, 10, r, nr, sums);
+    return sp_sums(c, u, 0, n0, n1, n2, axis, 1, s, false, 10, r, nr, sums);
 }
 
 }  // namespace fwt
