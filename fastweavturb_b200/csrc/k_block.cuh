@@ -235,8 +235,9 @@ __global__ void __launch_bounds__(kDepThreads, Policy::kCtas) deposit_block_kern
     float p0, p1;
     unpk(poison, p0, p1);
     if ((!(p0 == p0) || !(p1 == p1)) && !D.emit_only) atomicOr(err, 4);
-    nacc = __reduce_add_sync(0xffffffffu, nacc);   // a tile's pairs: at most 2^26 records x 1024 points / 8 warps
-    if (lane == 0 && tally && !D.emit_only && nacc) atomicAdd(tally, (unsigned long long)nacc);
+    // a lane's pairs: at most 2 points x 16 blocks x 2^26 records; the warp's do not fit 32 bits
+    const unsigned long long wacc = warp_sum((unsigned long long)nacc);
+    if (lane == 0 && tally && !D.emit_only && wacc) atomicAdd(tally, wacc);
     __syncthreads();
     if (S.failed && tid == 0) atomicOr(err, 2);
     if (D.emit_only) return;
