@@ -185,68 +185,105 @@ __global__ void fbb_bridge_kernel(uint64_t seed, int t0, int Np, int M, double d
 // takes two (its circulant row and its tubes), so a bound of eight made every plan anew in each call
 // of five or more levels.  Five levels of 4 x 256 to 1024 x 4096 nodes: 3.8-18 ms a call with plans
 // made anew, 0.96 ms with plans kept (0.36 of it fbb_fill_kernel's Gaussians, 0.24 the transforms, 0.14
-// fbb_bridge_kernel, 0.36 before it shared the bridge's powers).  At most 32 are kept; the oldest is
-// dropped.
+// fbb_bridge_kernel, 0.36 before it shared the bridge's powers).  Those are repeated shapes; where each
+// call draws other tube counts (3 to 6 levels, median of 100 calls) only the circulant rows' plans are met
+// again: 1.8 ms, 3.5 with eight plans.  A fresh context's first call makes all of its plans: 6 ms either
+// way.  At most 32 are kept; the oldest is dropped.
 constexpr size_t kFbbPlans = 32;
 
-static int fbb_plan(Ctx *c, int n2, int batch, cufftHandle *out)
+static int fbb_plan(Ctx *c, int n2, int batch, Ctx::FftPlan *out)
 {
-    const Ctx::FftPlan *f = nullptr;
     for (const auto &p : c->fbb_plans)
-        if (p.n2 == n2 && p.batch == batch) f = &p;
-    if (!f) {
-        if (c->fbb_plans.size() >= kFbbPlans) {
-            cufftDestroy(c->fbb_plans.front().h);
-            c->fbb_plans.erase(c->fbb_plans.begin());
+        if (p.n2 == n2 && p.batch == batch) {
+            *out = p;
+            return 0;
         }
-        cufftHandle h = 0;
-        int n[1] = {n2};
-        size_t ws = 0;
-        FWT_CUFFT(cufftCreate(&h));
-        cufftResult r = cufftSetAutoAllocation(h, 0);
-        if (r == CUFFT_SUCCESS) r = cufftMakePlanMany(h, 1, n, nullptr, 1, n2, nullptr, 1, n2, CUFFT_Z2Z, batch, &ws);
-        if (r != CUFFT_SUCCESS) cufftDestroy(h);
-        FWT_CUFFT(r);
-        c->fbb_plans.push_back({n2, batch, h, ws});
-        f = &c->fbb_plans.back();
+    if (c->fbb_plans.size() >= kFbbPlans) {
+        cufftDestroy(c->fbb_plans.front().h);
+        c->fbb_plans.erase(c->fbb_plans.begin());
     }
-    if (f->ws > c->fbb_ws_bytes) {
-        if (c->fbb_ws) cudaFree(c->fbb_ws);   // waits for the device
-        c->fbb_ws = nullptr;
-        c->fbb_ws_bytes = 0;
-        FWT_CUDA(cudaMalloc(&c->fbb_ws, f->ws));
-        c->fbb_ws_bytes = f->ws;
-    }
-    FWT_CUFFT(cufftSetStream(f->h, c->stream));
-    if (f->ws) FWT_CUFFT(cufftSetWorkArea(f->h, c->fbb_ws));
-    *out = f->h;
+    cufftHandle h = 0;
+    int n[1] = {n2};
+    size_t ws = 0;
+    FWT_CUFFT(cufftCreate(&h));
+    cufftResult r = cufftSetAutoAllocation(h, 0);
+    if (r == CUFFT_SUCCESS) r = cufftMakePlanMany(h, 1, n, nullptr, 1, n2, nullptr, 1, n2, CUFFT_Z2Z, batch, &ws);
+    if (r != CUFFT_SUCCESS) cufftDestroy(h);
+    FWT_CUFFT(r);
+    c->fbb_plans.push_back({n2, batch, h, ws});
+    *out = c->fbb_plans.back();
     return 0;
+}
+
+// The plans' work area, at least `bytes`.
+static int fbb_work_area(Ctx *c, size_t bytes)
+{
+    if (bytes <= c->fbb_ws_bytes) return 0;
+    if (c->fbb_ws) cudaFree(c->fbb_ws);   // waits for the device
+    c->fbb_ws = nullptr;
+    c->fbb_ws_bytes = 0;
+    const cudaError_t e = cudaMalloc(&c->fbb_ws, bytes);
+    if (e != cudaSuccess) {
+        c->fbb_ws = nullptr;
+        cudaGetLastError();
+        return fail(FWT_E_NOMEM, "generator: work area of " + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e));
+    }
+    c->fbb_ws_bytes = bytes;
+    return 0;
+}
+
+static int fbb_transform(Ctx *c, int n2, int batch, cufftDoubleComplex *data)
+{
+    Ctx::FftPlan p;
+    FWT_TRY(fbb_plan(c, n2, batch, &p));
+    FWT_TRY(fbb_work_area(c, p.ws));
+    FWT_CUFFT(cufftSetStream(p.h, c->stream));
+    if (p.ws) FWT_CUFFT(cufftSetWorkArea(p.h, c->fbb_ws));
+    FWT_CUFFT(cufftExecZ2Z(p.h, data, data, CUFFT_FORWARD));
+    return 0;
+}
+
+// Tubes of a batch: 3 complex rows of n2 per tube, ~1 GB per batch.
+static int fbb_batch(int T, int n2)
+{
+    return std::max(1, (int)std::min<int64_t>(T, ((int64_t)1 << 30) / ((int64_t)3 * n2 * 16)));
 }
 
 int fbb_generate(Ctx *c, uint64_t seed, int nlev, const int *tubes, const int *nodes, const double *H,
                  const double *dB, double *d_x, double *d_y, double *d_z)
 {
-    int64_t node0 = 0;
-    int t0 = 0;
+    // The call's plans first, and one work area for all of them: grown from level to level, which come in
+    // growing order, each growth waited for the device.  (What is beyond the plans kept grows below.)
+    size_t made = 0, ws = 0;
     for (int lv = 0; lv < nlev; ++lv) {
         const int T = tubes[lv], Np = nodes[lv];
         if (T < 0 || Np < 2) return fail(FWT_E_ARG, "generator: tubes >= 0 and nodes >= 2 required");
         if (!(H[lv] > 0 && H[lv] < 1)) return fail(FWT_E_ARG, "generator: H must be in (0,1)");
         if (Np < 128 && 128 % Np) return fail(FWT_E_ARG, "generator: nodes below 128 must divide 128");
+        const int n2 = 2 * (Np < 128 ? 128 : Np), per = fbb_batch(T, n2);
+        const int batch[3] = {1, T >= per ? 3 * per : 0, 3 * (T % per)};
+        for (int b : batch) {
+            if (b == 0 || ++made > kFbbPlans) continue;
+            Ctx::FftPlan p;
+            FWT_TRY(fbb_plan(c, n2, b, &p));
+            ws = std::max(ws, p.ws);
+        }
+    }
+    FWT_TRY(fbb_work_area(c, ws));
+    int64_t node0 = 0;
+    int t0 = 0;
+    for (int lv = 0; lv < nlev; ++lv) {
+        const int T = tubes[lv], Np = nodes[lv];
         const int M = Np < 128 ? 128 : Np, n2 = 2 * M;
         // eigenvalues of the circulant embedding
         FWT_TRY(buf_reserve(c, c->scratch[2], sizeof(cufftDoubleComplex) * n2 + sizeof(double) * n2));
         cufftDoubleComplex *row = (cufftDoubleComplex *)c->scratch[2].p;
         double *sq = (double *)(row + n2);
         fbb_row_kernel<<<(n2 + 255) / 256, 256, 0, c->stream>>>(M, H[lv], row);
-        cufftHandle p1;
-        FWT_TRY(fbb_plan(c, n2, 1, &p1));
-        FWT_CUFFT(cufftExecZ2Z(p1, row, row, CUFFT_FORWARD));
+        FWT_TRY(fbb_transform(c, n2, 1, row));
         fbb_sqrt_kernel<<<(n2 + 255) / 256, 256, 0, c->stream>>>(n2, Np, H[lv], row, sq);
         c->launches += 3;
-        // batches of tubes: 3 complex rows of n2 per tube, ~1 GB per batch
-        const int per = std::max(1, (int)std::min<int64_t>(T, ((int64_t)1 << 30) / ((int64_t)3 * n2 * 16)));
-        cufftHandle pb = 0;
+        const int per = fbb_batch(T, n2);
         for (int tb = 0; tb < T; tb += per) {
             const int nt = std::min(per, T - tb), nb = 3 * nt;
             FWT_TRY(buf_reserve(c, c->scratch[3], sizeof(cufftDoubleComplex) * (size_t)nb * n2));
@@ -255,8 +292,7 @@ int fbb_generate(Ctx *c, uint64_t seed, int nlev, const int *tubes, const int *n
             double *fbm = (double *)c->scratch[4].p;
             const int64_t tot = (int64_t)nb * n2;
             fbb_fill_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(seed, t0 + tb, nb, n2, sq, Zb);
-            FWT_TRY(fbb_plan(c, n2, nb, &pb));
-            FWT_CUFFT(cufftExecZ2Z(pb, Zb, Zb, CUFFT_FORWARD));
+            FWT_TRY(fbb_transform(c, n2, nb, Zb));
             fbb_scan_kernel<<<nb, 256, 0, c->stream>>>(Zb, n2, M, fbm);
             fbb_bridge_kernel<<<nt, 256, 0, c->stream>>>(seed, t0 + tb, Np, M, dB[lv], row, fbm, d_x, d_y, d_z,
                                                          node0 + (int64_t)tb * Np);
