@@ -155,24 +155,33 @@ __device__ __forceinline__ float turning_integrand(const float (&d1)[3][5], cons
 //   4. section_fp64_kernel  one warp per listed section: the reference's sum in FP64
 // Bound by FP32 issue: step 3 takes 1500 warp instructions a section, step 1 about 110.  With every
 // section in step 3 (and 4) the 38 M sections of a six-level field (H = 0.7) took 68 ms; the four
-// together take 9.7 ms (5.6, 2.5, 1.0, 0.6).
+// together take 10.0 ms (5.8, 2.6, 1.0, 0.6).
 //
-// The bound.  With h the sample spacing, the trapezoidal sum of a smooth integrand f is off by
-// about h / 12 sum |second differences of f|, and so is that of a kink (|c' x c''| passing near
-// zero) or of any feature wider than h; Simpson's rule, which is used, is rarely off by as much.
-// What the samples cannot show is a peak of 1 / |c'|^2 between two of them: a zero of the positive
-// polynomial |c'|^2 at a distance b from the section in the complex plane gives |c'|^2 a second
-// difference of 2 h^2 / (d^2 + b^2) of itself at a sample d <= h / 2 away, so where no second
-// difference exceeds a tenth of |c'|^2 every b is above 4 h and the peaks are resolved; where one
-// does, the section counts as undecided.  Twice the bound is allowed for: over 1.1 M sections of
-// fractional bridges with H from 0.3 to 0.8 the sum's distance from the reference's stayed below
-// 0.47 of it.  The reference's sum itself is a trapezoidal sum with ntf_pre intervals plus half the
-// end values: ntf_pre >= 512 keeps its own distance from the integral far below the bound; smaller
-// values go to step 3 at once.
+// The bound.  Simpson's rule over 2h is off by the integral of f'' times a kernel that is at most h^2/6,
+// and a second difference is h f'' averaged over a hat of that width: h / 6 sum |second differences|
+// bounds the error of the integrand f, kinks included (|c' x c''| passing near zero), as long as f'' keeps
+// its sign within a spacing.  What the samples cannot show is a peak of 1 / |c'|^2 between two of them: a
+// zero of the positive polynomial |c'|^2 at a distance b from the section in the complex plane gives |c'|^2
+// a second difference of 2 h^2 / (d^2 + b^2) of itself at a sample d <= h / 2 away, so where no second
+// difference exceeds a tenth of |c'|^2 a single zero is beyond 4 h and its peak is resolved; where one
+// does, the section counts as undecided.  This is an argument, not a proof (f'' may change sign between
+// samples, zeros may offset each other), so it was measured: over 1.9 G sections, the 1.23 G of an
+// eight-level field of 1024^3 and 0.7 G of fractional bridges with H from 0.3 to 0.9, the sum's distance
+// from the reference's stayed below 0.62 of the bound (beyond half of it in one section in a million), and no
+// section got another count than from step 3 alone.  A miss would cost that section one sub-segment more
+// or less.  The reference's sum itself is a trapezoidal sum with ntf_pre intervals plus half the end
+// values: ntf_pre >= 512 keeps its own distance from the integral far below the bound; smaller values go
+// to step 3 at once.
+//
+// The rounding.  FP32 sums run over at most 32 samples and are added in FP64, in steps 1, 2 and 3 alike;
+// 1e-4 of the result is allowed for the FP32 integrand.  Next to a cusp (|c'| close to zero) step 3's
+// integrand can be off by more: 11 of those 1.23 G sections, and 32 of the 0.7 G, differ by one
+// sub-segment from the reference's sum in FP64.
 constexpr int kQuadMinPre = 512;
 
 struct SectionSum {
-    float tsum, err;   // sum over the reference's samples (without the step), bound of its error
+    double tsum;   // sum over the reference's samples (without the step)
+    float err;     // bound of its error
     bool resolved;
 };
 
@@ -184,7 +193,8 @@ __device__ __forceinline__ SectionSum section_quadrature(const float (&d1)[3][5]
     float q0, q1, q2;
     float f0 = turning_integrand(d1, d2, 0.0f, q0), f1 = turning_integrand(d1, d2, dz, q1);
     const float fa = f0, qa = q0;
-    float odd = f1, even = 0.0f, dd = 0.0f;   // interior sums, sum of |second differences|
+    double sum = 0.0;                         // 4 x odd + 2 x even samples
+    float odd = f1, even = 0.0f, dd = 0.0f;   // of up to 32 of them; sum of |second differences|
     float qx = 0.0f;                          // the first end's second difference
     bool rough = false;
 #pragma unroll 2
@@ -198,6 +208,10 @@ __device__ __forceinline__ SectionSum section_quadrature(const float (&d1)[3][5]
         if (i < Intervals) {
             if (i & 1) odd += f2;
             else even += f2;
+            if (i % 32 == 31) {
+                sum += 4.0 * (double)odd + 2.0 * (double)even;
+                odd = even = 0.0f;
+            }
         }
         f0 = f1;
         f1 = f2;
@@ -207,7 +221,8 @@ __device__ __forceinline__ SectionSum section_quadrature(const float (&d1)[3][5]
     rough = rough || !(qx <= 0.1f * qa);
     SectionSum s;
     // n_pre times Simpson's integral over the unit interval, plus half the end values
-    s.tsum = fmaf((fa + f1 + 4.0f * odd + 2.0f * even) * (h / 3.0f), (float)ntf_pre, 0.5f * (fa + f1));
+    const double ends = (double)fa + (double)f1;
+    s.tsum = (ends + sum) * ((double)ntf_pre / (3.0 * Intervals)) + 0.5 * ends;
     s.err = (2.0f / 12.0f) * h * dd * (float)ntf_pre;
     s.resolved = !rough;
     return s;
@@ -218,7 +233,7 @@ __device__ __forceinline__ SectionSum section_quadrature(const float (&d1)[3][5]
 __device__ __forceinline__ int section_decide(const SectionSum &q, double dtfp, double L, int ntf_times, int &ntf)
 {
     const double k = dtfp * L * ntf_times / dev_pi2();
-    const double x = (double)q.tsum * k, rounding = 1e-4 * (x + 1.0), e = (double)q.err * k;
+    const double x = q.tsum * k, rounding = 1e-4 * (x + 1.0), e = (double)q.err * k;
     if (!q.resolved || !(x == x) || !(e == e)) return 1;
     const double m = e + rounding;
     if (floor(x + m) == floor(x - m)) {
