@@ -173,10 +173,10 @@ __device__ __forceinline__ float turning_integrand(const float (&d1)[3][5], cons
 // values: ntf_pre >= 512 keeps its own distance from the integral far below the bound; smaller values go
 // to step 3 at once.
 //
-// The rounding.  FP32 sums run over at most 32 samples and are added in FP64, in steps 1, 2 and 3 alike;
-// 1e-4 of the result is allowed for the FP32 integrand.  Next to a cusp (|c'| close to zero) step 3's
-// integrand can be off by more: 11 of those 1.23 G sections, and 32 of the 0.7 G, differ by one
-// sub-segment from the reference's sum in FP64.
+// The rounding.  FP32 sums run over at most 32 samples (in step 3 a lane's ntf_pre / 32, in two sums) and
+// are added in FP64; 1e-4 of the result is allowed for the FP32 integrand.  Next to a cusp (|c'| close to
+// zero) step 3's integrand can be off by more: 11 of those 1.23 G sections, and 32 of the 0.7 G, have
+// another count than by the reference's sum in FP64.
 constexpr int kQuadMinPre = 512;
 
 struct SectionSum {
