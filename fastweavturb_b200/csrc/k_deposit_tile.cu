@@ -215,63 +215,68 @@ constexpr uint32_t kQDecide = 1u << 15;
 // Pairs whose curved-branch amplification exceeds kRedoCond, and pairs with a plane test
 // within its rounding bound (kQDecide), are deferred to FP64 (DeferList) instead.  In the
 // emit-only pass (D.emit_only) nothing is added and only the deferred pairs are listed again.
+// General = false (constant cores without a twist) is an FP64 form only: in FP32 such lines take
+// deposit_block_kernel.
 template <bool General, bool F64>
 __device__ __forceinline__ void drain_queue(WarpStage &S, long long (*acc)[kAccN], int lane, int cnt, int &qn,
                                             unsigned &nacc, float fscale, float fmaxq, int *__restrict__ err,
                                             const RedoCtx &redo, const DeferList &D, int x0, int y0, int z0)
 {
-    bool flag = false, ok64 = false, counted = false;
-    uint32_t rrec = 0;
-    int lx = 0, ly = 0, lz = 0;
-    if (F64 && lane < cnt) {
-        // FP64 tile path: the candidate passed the widened FP32 tests; the reference's FP64
-        // tests decide, at its index in the sub-segment's own box
-        const uint32_t e = S.q[lane];
-        const int k = (int)(e & 15u);
-        lx = (int)((e >> 4) & 15u), ly = (int)((e >> 8) & 7u), lz = (int)((e >> 11) & 7u);
-        const CandBox &B = S.box[k];
-        const SegRec &R = S.rec[k];
-        ok64 = eval_pair_f64<General>(redo, (int64_t)(S.id[k] & ((1u << 26) - 1u)), R.box_lo[0] + lx + B.dl[0],
-                      R.box_lo[1] + ly + B.dl[1], R.box_lo[2] + lz + B.dl[2], reinterpret_cast<double(*)[kAccN]>(acc),
-                      lx + kSY * ly + kSZ * lz);
-    } else if (lane < cnt) {
-        const uint32_t e = S.q[lane];
-        const int k = (int)(e & 15u);
-        lx = (int)((e >> 4) & 15u), ly = (int)((e >> 8) & 7u), lz = (int)((e >> 11) & 7u);
-        if (e & kQDecide) {
-            flag = true;
-            rrec = (S.id[k] & ((1u << 26) - 1u)) | kDeferDecide;
-        } else if (General || !D.emit_only) {
-            counted = true;
+    static_assert(General || F64, "FP32 lines of constant cores take deposit_block_kernel");
+    if constexpr (F64) {
+        bool ok64 = false;
+        if (lane < cnt) {
+            // the candidate passed the widened FP32 tests; the reference's FP64 tests decide, at its
+            // index in the sub-segment's own box
+            const uint32_t e = S.q[lane];
+            const int k = (int)(e & 15u);
+            const int lx = (int)((e >> 4) & 15u), ly = (int)((e >> 8) & 7u), lz = (int)((e >> 11) & 7u);
             const CandBox &B = S.box[k];
             const SegRec &R = S.rec[k];
-            const float d0x = fmaf((float)(lx + B.dl[0]), R.dx, R.off[0]);
-            const float d0y = fmaf((float)(ly + B.dl[1]), R.dx, R.off[1]);
-            const float d0z = fmaf((float)(lz + B.dl[2]), R.dx, R.off[2]);
-            // the pair passed rec_classify: only t0 (the spline argument) is needed again
-            const float t0 = fmaf(d0z, R.tc0[2], fmaf(d0y, R.tc0[1], d0x * R.tc0[0]));
-            float vv[3], cond;
-            rec_vorticity<General>(R, d0x, d0y, d0z, t0, vv, cond);
-            const int p = lx + kSY * ly + kSZ * lz;
-            flag = General && !(cond <= kRedoCond);
-            if (flag) {
-                rrec = S.id[k] & ((1u << 26) - 1u);
-            } else if (!D.emit_only) {
+            ok64 = eval_pair_f64<General>(redo, (int64_t)(S.id[k] & ((1u << 26) - 1u)), R.box_lo[0] + lx + B.dl[0],
+                                          R.box_lo[1] + ly + B.dl[1], R.box_lo[2] + lz + B.dl[2],
+                                          reinterpret_cast<double(*)[kAccN]>(acc), lx + kSY * ly + kSZ * lz);
+        }
+        nacc += __popc(__ballot_sync(0xffffffffu, ok64));
+    } else {
+        bool flag = false, counted = false;
+        uint32_t rrec = 0;
+        int lx = 0, ly = 0, lz = 0;
+        if (lane < cnt) {
+            const uint32_t e = S.q[lane];
+            const int k = (int)(e & 15u);
+            lx = (int)((e >> 4) & 15u), ly = (int)((e >> 8) & 7u), lz = (int)((e >> 11) & 7u);
+            if (e & kQDecide) {
+                flag = true;
+                rrec = (S.id[k] & ((1u << 26) - 1u)) | kDeferDecide;
+            } else {
+                counted = true;
+                const CandBox &B = S.box[k];
+                const SegRec &R = S.rec[k];
+                const float d0x = fmaf((float)(lx + B.dl[0]), R.dx, R.off[0]);
+                const float d0y = fmaf((float)(ly + B.dl[1]), R.dx, R.off[1]);
+                const float d0z = fmaf((float)(lz + B.dl[2]), R.dx, R.off[2]);
+                // the pair passed rec_classify: only t0 (the spline argument) is needed again
+                const float t0 = fmaf(d0z, R.tc0[2], fmaf(d0y, R.tc0[1], d0x * R.tc0[0]));
+                float vv[3], cond;
+                rec_vorticity<true>(R, d0x, d0y, d0z, t0, vv, cond);
+                const int p = lx + kSY * ly + kSZ * lz;
+                flag = !(cond <= kRedoCond);
+                if (flag) {
+                    rrec = S.id[k] & ((1u << 26) - 1u);
+                } else if (!D.emit_only) {
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    float sv = vv[d] * fscale;
-                    if (!(fabsf(sv) < fmaxq)) {
-                        atomicOr(err, 4);
-                        sv = sv != sv ? 0.0f : copysignf(fmaxq, sv);
+                    for (int d = 0; d < 3; ++d) {
+                        float sv = vv[d] * fscale;
+                        if (!(fabsf(sv) < fmaxq)) {
+                            atomicOr(err, 4);
+                            sv = sv != sv ? 0.0f : copysignf(fmaxq, sv);
+                        }
+                        atomicAdd((unsigned long long *)&acc[d][p], (unsigned long long)__float2ll_rn(sv));
                     }
-                    atomicAdd((unsigned long long *)&acc[d][p], (unsigned long long)__float2ll_rn(sv));
                 }
             }
         }
-    }
-    if constexpr (F64) {
-        nacc += __popc(__ballot_sync(0xffffffffu, ok64));
-    } else {
         nacc += __popc(__ballot_sync(0xffffffffu, counted));
         defer_push(D, lane, flag, rrec, x0 + lx, y0 + ly, z0 + lz);
     }
