@@ -182,7 +182,10 @@ void buf_free(Ctx *c, DevBuf &b);
 
 // centerline set-up + deposition (k_centerline.cu, k_deposit.cu)
 int deposit_lines(Ctx *c, int line_s, int line_e);
-int side_fold(Ctx *c);   // add the deferred pairs' sums into omega (k_deposit_tile.cu)
+// the side accumulator (int64 sums beside omega), allocated and zeroed on first use, and its sums added
+// into omega (k_deposit_tile.cu)
+int side_ensure(Ctx *c);
+int side_fold(Ctx *c);
 
 // spectral (k_spectral.cu)
 int spectral_init(Ctx *c);

@@ -183,8 +183,7 @@ int deposit_lines(Ctx *c, int line_s, int line_e)
     // FWT_SCATTER_RT_CELLS, else the default
     const char *senv = std::getenv("FWT_SCATTER_RT_CELLS");
     const double sca_cells =
-        c->scatter_rt_cells >= 0.0 ? c->scatter_rt_cells
-                                   : (senv ? std::atof(senv) : kScatterMaxRtCells);
+        c->scatter_rt_cells >= 0.0 ? c->scatter_rt_cells : (senv ? std::atof(senv) : kScatterMaxRtCells);
     auto scattered = [&](int l) {
         return thin(l) && c->p.precision == 32 && !rasterised(l) &&
                c->p.Rtube_ratio * c->p.sigma_ratio * c->sigma[l] <= sca_cells * dxg;
@@ -237,6 +236,13 @@ int deposit_lines(Ctx *c, int line_s, int line_e)
             FWT_TRY(launch_walk(c, B, d_acc));
         } else {
             int64_t np_ = 0;
+            if (B.scatter) {
+                // 32 bytes a grid point, which the tiles need only where a pair is handed to FP64: lines
+                // for which there is no room go through the tiles
+                const int rc = side_ensure(c);
+                if (rc == FWT_E_NOMEM) B.scatter = false;
+                else FWT_TRY(rc);
+            }
             if (mode == BatchRecords::Pieces && B.scatter) FWT_TRY(launch_scatter(c, B));
             else if (mode == BatchRecords::Pieces) FWT_TRY(launch_piece(c, B, &np_));
             else FWT_TRY(launch_tile(c, B, &np_));

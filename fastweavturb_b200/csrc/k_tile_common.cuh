@@ -449,8 +449,6 @@ RedoCtx redo_ctx(const Ctx *c, const CenterlineBatch &B, double scale, bool piec
 // The deferred-pair list of a launch over `units` work units ((tile, record) pairs, or pieces),
 // sized from the running rate of deferred pairs per unit (k_deposit_tile.cu).
 int defer_list(Ctx *c, int64_t units, double rate, DeferList &D);
-// The side accumulator (kSideStride int64 per grid point), allocated and zeroed on first use.
-int side_ensure(Ctx *c);
 
 // Evaluate the first n pairs of the list in FP64 into the side accumulator (k_deposit_tile.cu).
 int defer_apply(Ctx *c, const RedoCtx &R, const DeferList &D, unsigned long long n);

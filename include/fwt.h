@@ -254,8 +254,8 @@ int fwt_counters(fwt_ctx *ctx, int64_t *c, int n);
  * `value` grid spacings are deposited without tiles: each piece is searched once and its
  * contributions are added as int64 fixed point with global reductions (the sums do not depend
  * on the order); thicker piece lines go through the tiles.  0 switches it off, value < 0
- * restores the default, 8.  The field is the same
- * either way to FP32 rounding. */
+ * restores the default, 8.  Where its sums (32 bytes a grid point) do not fit the memory or its
+ * cap, the lines go through the tiles too.  The field is the same either way to FP32 rounding. */
 #define FWT_TUNE_SCATTER_RT_CELLS 3
 /* FWT_TUNE_DEFER_MAX_PAIRS: the most entries (16 bytes each) the list of pairs an FP32 launch
  * hands to FP64 grows to after an overflow; a launch that hands over more lists and evaluates
