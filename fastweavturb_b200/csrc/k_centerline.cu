@@ -148,7 +148,8 @@ __device__ __forceinline__ float turning_integrand(const float (&d1)[3][5], cons
 // samples (1001): ntf = ceil(ntf_times theta / 2 pi) + 1, an integer, so theta is needed only well
 // enough to tell which step of ceil it falls on.  The sections (n_sec + 1 slots per line; slot
 // n_sec is the periodic copy) are decided by ever finer quadratures, each with a bound on its
-// error; a section whose bound straddles a step goes to the next one's list:
+// error; a section whose bound straddles a step goes to the next one's list (section_coarse leaves steps
+// out where there are few sections):
 //   1. section_coe_kernel   one thread per section: coefficients (FP64), 64 intervals
 //   2. section_fine_kernel  one thread per listed section: 256 intervals
 //   3. section_kernel       one warp per listed section: the reference's own sum in FP32
@@ -178,6 +179,17 @@ __device__ __forceinline__ float turning_integrand(const float (&d1)[3][5], cons
 // zero) step 3's integrand can be off by more: 11 of those 1.23 G sections, and 32 of the 0.7 G, have
 // another count than by the reference's sum in FP64.
 constexpr int kQuadMinPre = 512;
+
+// Quadratures before step 3: 0 none, 1 the 64 intervals, 2 both.  A thread walks its intervals in a
+// chain, 5 us for 64 of them and 20 for 256 however few sections there are, while step 3 has a warp for
+// each: few sections go to it at once.  All steps, us, with 0 / 1 / 2 (fractional bridges, H = 0.3):
+// 1,028 slots 30 / 35 / 58, 4,112 44 / 45 / 66, 16,448 64 / 50 / 69, 65,792 161 / 80 / 84, 131,584
+// 293 / 125 / 110.
+inline int section_coarse(int ntf_pre, int64_t slots)
+{
+    if (ntf_pre < kQuadMinPre || slots <= (1 << 12)) return 0;
+    return slots <= (1 << 16) ? 1 : 2;
+}
 
 struct SectionSum {
     double tsum;   // sum over the reference's samples (without the step)
@@ -266,8 +278,8 @@ __global__ void __launch_bounds__(256) section_coe_kernel(
     const LineParam *__restrict__ lp, const int *__restrict__ slot_line, int64_t nslots, const double *__restrict__ X,
     const double *__restrict__ Y, const double *__restrict__ Z, const double *__restrict__ cze,
     const double *__restrict__ ck, const double *__restrict__ ckk, const double *__restrict__ Len, int64_t node_base,
-    int ntf_times, int ntf_pre, double *__restrict__ coe_out, float *__restrict__ zstep_out, int *__restrict__ ntf_out,
-    double *__restrict__ dtf_out, const SectionLists lists)
+    int ntf_times, int ntf_pre, int coarse, double *__restrict__ coe_out, float *__restrict__ zstep_out,
+    int *__restrict__ ntf_out, double *__restrict__ dtf_out, const SectionLists lists)
 {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nslots) return;
@@ -312,11 +324,11 @@ __global__ void __launch_bounds__(256) section_coe_kernel(
     const double dtfp = (zr_ - zl) / (1.0 * ntf_pre);
     zstep_out[s] = (float)(dtfp * L);
     int left = 1, ntf = 0;
-    if (ntf_pre >= kQuadMinPre)
+    if (coarse > 0)
         left = section_decide(section_quadrature<64>(d1, d2, (float)zr, ntf_pre), dtfp, L, ntf_times, ntf);
     ntf_out[s] = ntf;
     dtf_out[s] = left == 0 ? (zr_ - zl) / (1.0 * ntf) : 0.0;
-    const bool fine = left == 1 && ntf_pre >= kQuadMinPre;
+    const bool fine = left == 1 && coarse > 1;
     list_push(lists.count, lists.fine, fine, (unsigned)s);
     list_push(lists.count + 1, lists.full, left == 1 && !fine, (unsigned)s);
     list_push(lists.count + 2, lists.fp64, left == 2, (unsigned)s);
@@ -995,19 +1007,22 @@ int centerline_setup(Ctx *c, int la, int lb, CenterlineBatch &B, BatchRecords mo
     FWT_TRY(buf_reserve(c, C.scratch[28], sizeof(float) * (size_t)std::max<int64_t>(slots, 1)));
     float *d_zstep = (float *)C.scratch[28].p;
     const unsigned tblocks = (unsigned)((slots + 255) / 256);
+    const int coarse = section_coarse(c->p.ntf_pre, slots);
     section_coe_kernel<<<tblocks, 256, 0, c->stream>>>(B.lp, B.slot_line, slots, c->d_x, c->d_y, c->d_z, B.cze, B.ck,
-                                                      B.ckk, B.Len, B.node_base, c->p.ntf_times, c->p.ntf_pre, B.coe,
-                                                      d_zstep, B.ntf, B.dtf, lists);
+                                                      B.ckk, B.Len, B.node_base, c->p.ntf_times, c->p.ntf_pre, coarse,
+                                                      B.coe, d_zstep, B.ntf, B.dtf, lists);
     // fixed grids over the lists, no larger than the slots
-    const unsigned fblocks = (unsigned)std::min<int64_t>((slots + 127) / 128, 148 * 8);
-    section_fine_kernel<<<fblocks, 128, 0, c->stream>>>(B.lp, B.slot_line, B.cze, B.Len, B.node_base, c->p.ntf_times,
-                                                       c->p.ntf_pre, B.coe, B.ntf, B.dtf, lists);
+    if (coarse > 1) {
+        const unsigned fblocks = (unsigned)std::min<int64_t>((slots + 127) / 128, 148 * 8);
+        section_fine_kernel<<<fblocks, 128, 0, c->stream>>>(B.lp, B.slot_line, B.cze, B.Len, B.node_base, c->p.ntf_times,
+                                                           c->p.ntf_pre, B.coe, B.ntf, B.dtf, lists);
+    }
     const unsigned wgrid = (unsigned)std::min<int64_t>((slots + 7) / 8, 148 * 8);
     section_kernel<<<wgrid, 256, 0, c->stream>>>(B.lp, B.slot_line, B.cze, B.Len, B.node_base, c->p.ntf_times,
                                                  c->p.ntf_pre, B.coe, d_zstep, B.ntf, B.dtf, lists);
     section_fp64_kernel<<<(unsigned)std::min<int64_t>((slots + 7) / 8, 4 * 148), 256, 0, c->stream>>>(
         B.lp, B.slot_line, B.cze, B.Len, B.node_base, c->p.ntf_times, c->p.ntf_pre, B.coe, B.ntf, B.dtf, lists);
-    c->launches += 4;
+    c->launches += 3 + (coarse > 1);
     kt_end(c, km);
     km = kt_begin(c, KT_CENTERLINE);
     slot_counts_kernel<<<(unsigned)((slots + 255) / 256), 256, 0, c->stream>>>(B.lp, B.slot_line, slots, B.ntf,
