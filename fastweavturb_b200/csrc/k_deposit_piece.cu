@@ -1262,7 +1262,7 @@ __device__ __forceinline__ void scatter_drain(ScatterStage &S, int lane, int cnt
 
 template <bool General>
 __global__ void __launch_bounds__(kScatterWarps * 32, 3) scatter_piece_kernel(
-    const PieceRec *__restrict__ rec, int64_t npieces, int N, int zs, int nz, float fscale,
+    const PieceRec *__restrict__ rec, int64_t npieces, int per, int N, int zs, int nz, float fscale,
     unsigned long long *__restrict__ side, int prefetch, int *__restrict__ err, const DeferList D,
     unsigned long long *__restrict__ tally)
 {
@@ -1270,13 +1270,14 @@ __global__ void __launch_bounds__(kScatterWarps * 32, 3) scatter_piece_kernel(
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
     ScatterStage &S = reinterpret_cast<ScatterStage *>(dsm)[warp];
-    const int64_t nchunks = (npieces + kPChunk - 1) / kPChunk;
+    const int64_t nchunks = (npieces + per - 1) / per;
     const int64_t nw = (int64_t)gridDim.x * kScatterWarps;
     unsigned long long nacc = 0;   // pairs evaluated by this warp (warp-uniform)
     const int64_t chend = min(nchunks, (int64_t)D.w1);
-    for (int64_t ch = (int64_t)D.w0 + (int64_t)blockIdx.x * kScatterWarps + warp; ch < chend; ch += nw) {
-        const int64_t p0 = ch * kPChunk;
-        const int nc = (int)min((int64_t)kPChunk, npieces - p0);
+    // neighbouring chunks go to different blocks, so that few of them still reach every SM
+    for (int64_t ch = (int64_t)D.w0 + (int64_t)warp * gridDim.x + blockIdx.x; ch < chend; ch += nw) {
+        const int64_t p0 = ch * per;
+        const int nc = (int)min((int64_t)per, npieces - p0);
         {   // stage the chunk's records: coalesced 16-byte loads
             const uint4 *src = reinterpret_cast<const uint4 *>(rec + p0);
             uint4 *dst = reinterpret_cast<uint4 *>(S.rec);
@@ -1578,6 +1579,16 @@ int launch_piece(Ctx *c, const CenterlineBatch &B, int64_t *pairs_out)
     return 0;
 }
 
+// Pieces of a warp's chunk in scatter_piece_kernel: four (32 chords, one to a lane) where the pieces are
+// enough for the warps the chip holds, fewer where warps would have none.  One line of 64 nodes with a
+// twist, radius 7.9, a whole deposition: in chunks of four, eight to a block, 1.10 ms on 128^3 and 1.79 on
+// 256^3 (in tiles 0.91 and 1.49); spread out 0.73 and 1.17.
+static int scatter_pieces(int64_t npieces, int sms)
+{
+    const int64_t warps = (int64_t)sms * 3 * kScatterWarps;
+    return (int)std::min<int64_t>(kPChunk, (npieces + warps - 1) / warps);
+}
+
 int launch_scatter(Ctx *c, const CenterlineBatch &B)
 {
     if (B.npieces == 0) return 0;
@@ -1595,7 +1606,8 @@ int launch_scatter(Ctx *c, const CenterlineBatch &B)
     const int zs = c->slab_nz ? c->slab_z0 : 0, nz = c->slab_nz ? c->slab_nz : N;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
-    const int64_t nchunks = (B.npieces + kPChunk - 1) / kPChunk;
+    const int per = scatter_pieces(B.npieces, sms);
+    const int64_t nchunks = (B.npieces + per - 1) / per;
     unsigned long long *side = (unsigned long long *)c->b_side.p;
     // sums beyond the L2: fetched ahead of their additions (see scatter_drain)
     int l2 = 0;
@@ -1605,18 +1617,18 @@ int launch_scatter(Ctx *c, const CenterlineBatch &B)
     FWT_TRY(defer_list(c, B.npieces, c->defer_per_piece, D));
     auto launch = [&](const DeferList &L) -> int {
         const int64_t nch = std::min<int64_t>(nchunks, L.w1) - L.w0;
-        const unsigned grid = (unsigned)std::min<int64_t>((int64_t)sms * 3, (nch + kScatterWarps - 1) / kScatterWarps);
+        const unsigned grid = (unsigned)std::min<int64_t>((int64_t)sms * 3, nch);
         const int m = kt_begin(c, KT_DEPOSIT);
         if (general) {
             FWT_CUDA(cudaFuncSetAttribute(scatter_piece_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)kScatterSmem));
             scatter_piece_kernel<true><<<grid, kScatterWarps * 32, kScatterSmem, c->stream>>>(
-                B.piece, B.npieces, N, zs, nz, (float)scale, side, prefetch, d_err, L, rctx.tally);
+                B.piece, B.npieces, per, N, zs, nz, (float)scale, side, prefetch, d_err, L, rctx.tally);
         } else {
             FWT_CUDA(cudaFuncSetAttribute(scatter_piece_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)kScatterSmem));
             scatter_piece_kernel<false><<<grid, kScatterWarps * 32, kScatterSmem, c->stream>>>(
-                B.piece, B.npieces, N, zs, nz, (float)scale, side, prefetch, d_err, L, rctx.tally);
+                B.piece, B.npieces, per, N, zs, nz, (float)scale, side, prefetch, d_err, L, rctx.tally);
         }
         FWT_CUDA(cudaGetLastError());
         kt_end(c, m);
