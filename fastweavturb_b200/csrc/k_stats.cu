@@ -9,6 +9,7 @@
 #include "k_common.cuh"
 
 #include <cmath>
+#include <type_traits>
 
 namespace fwt {
 
@@ -138,15 +139,23 @@ __global__ void __launch_bounds__(256) pdf_kernel(const Real *__restrict__ a, si
 // for p <= 6, 14 for 10, where a running power took 21), the scale s = 1/u' enters as the power of
 // two just above it, exactly, when the lines are staged, and as the remainder in [0.5, 1) at the end,
 // only as many orders as asked for are summed, and separations equal modulo N once (the host's list).  512^3, three
-// components, orders 1-6: 14.5 ms with the running power to order 10, 7.8 now; at the FP64 rate
+// components, orders 1-6: 14.5 ms with the running power to order 10, 6.8 now; at the FP64 rate
 // the 17 separations take 3.8.
 template <typename Real>
 __host__ __device__ constexpr int sp_lines(int N)
 {
     return N < (sizeof(Real) == 8 ? 16 : 32) ? N : (sizeof(Real) == 8 ? 16 : 32);
 }
-constexpr int kSpPerWarp = 4;   // separations of a warp
-constexpr int kSpGroups = 8, kSpMaxThreads = 384;   // groups of separations in a block; six of them twice
+constexpr int kSpPerWarp = 4;   // separations of a warp at the most
+static_assert(kSpPerWarp == 4, "sp_kernel's loops");
+// Groups of separations in a block, and its threads.  The groups are spread evenly over as few blocks as
+// hold them, a group takes three or four separations (fewer only where there are fewer), and few groups
+// share the positions among several warps each.  With up to eight groups in the first block, four
+// separations in each whether asked for or not, and two warps a group, few separations took longer than
+// with one warp for every eighth: 512^3, ms (and with running powers): one separation, orders
+// 1-6: 7.9 -> 1.7 (5.3), 33, orders 1-10: 34.3 -> 21.2 (28.7), 17, orders 1-6: 7.8 -> 6.8 (13.6).
+constexpr int kSpGroups = 8, kSpMaxThreads = 384;
+constexpr int kSpPositions = 16;   // positions a lane at the least, where positions are shared
 
 template <int PMAX>
 __device__ __forceinline__ void sp_accumulate(double d, double (&acc)[PMAX])
@@ -177,14 +186,13 @@ __device__ __forceinline__ void sp_accumulate(double d, double (&acc)[PMAX])
 // The field is a box n0 x n1 x n2 (x fastest) whose extent along the axis is the line length N:
 // the whole grid, or a z-slab (axes 0, 1) or y-pencil (axis 2) of a grid split over GPUs.  The
 // axis is axis0 + blockIdx.y, its component stride elements further on per step.  blockDim is
-// 32 x (groups of separations) x (1 or 2 shares of the positions).
-// Groups beyond eight go to blockIdx.z.  Scaled: each increment is multiplied by `post` in FP64, for a
+// 32 x (groups of separations) x (shares of the positions); blockIdx.z takes the next groups.  Scaled: each increment is multiplied by `post` in FP64, for a
 // scale that says nothing about the field's size (a caller's own, or one beyond the staged type's
 // exponents), where sc is 1.
 template <typename Real, int PMAX, bool Scaled = false>
 __global__ void __launch_bounds__(kSpMaxThreads, PMAX > 6 ? 1 : 2) sp_kernel(const Real *__restrict__ u0, size_t stride, int N, int n0, int n1, int n2,
                                                  int axis0, Real sc, double post, const int *__restrict__ rs,
-                                                 int nr, double *__restrict__ Sp)
+                                                 int nr, int ngroups, double *__restrict__ Sp)
 {
     extern __shared__ __align__(16) unsigned char sp_smem[];
     Real *tile = reinterpret_cast<Real *>(sp_smem);   // N x (W + 1)
@@ -193,8 +201,9 @@ __global__ void __launch_bounds__(kSpMaxThreads, PMAX > 6 ? 1 : 2) sp_kernel(con
     const int W = sp_lines<Real>(N);
     const int ld = W + 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int all = (nr + kSpPerWarp - 1) / kSpPerWarp, ngroups = min(kSpGroups, all);
-    const int group = (int)blockIdx.z * kSpGroups + warp % ngroups;
+    // group g of all takes separations g, g + all, ...: four at the most, and none one more than another
+    const int all = ngroups * (int)gridDim.z, group = (int)blockIdx.z * ngroups + warp % ngroups;
+    const int count = group < nr ? (nr - 1 - group) / all + 1 : 0;
     // a lane's line, and the share of the positions that its part of the warp and its warp take
     const int per = 32 / W, line = lane % W, sub = lane / W;
     const int first = (warp / ngroups) * per + sub, pstep = (nwarps / ngroups) * per;
@@ -204,8 +213,7 @@ __global__ void __launch_bounds__(kSpMaxThreads, PMAX > 6 ? 1 : 2) sp_kernel(con
     for (int a = 0; a < kSpPerWarp; ++a) {
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) acc[a][p] = 0.0;
-        const int m = group * kSpPerWarp + a;
-        rr[a] = m < nr ? rs[m] : 0;   // a separation of zero adds zeros
+        rr[a] = a < count ? rs[group + a * all] : 0;
     }
     // axis 0: groups of W consecutive x-rows (row = y + n1 z); axes 1, 2: groups of W
     // consecutive x at fixed z (axis 1) or fixed y (axis 2)
@@ -232,26 +240,44 @@ __global__ void __launch_bounds__(kSpMaxThreads, PMAX > 6 ? 1 : 2) sp_kernel(con
         }
         __syncthreads();
         if (line < nl && sub < per) {
-            for (int pos = first; pos < N; pos += pstep) {
-                const double c = (double)tile[pos * ld + line];
+            auto run = [&](auto n) {
+                for (int pos = first; pos < N; pos += pstep) {
+                    const double c = (double)tile[pos * ld + line];
 #pragma unroll
-                for (int a = 0; a < kSpPerWarp; ++a) {
-                    int q = pos + rr[a];
-                    if (q >= N) q -= N;
-                    const double d = (double)tile[q * ld + line] - c;
-                    sp_accumulate<PMAX>(Scaled ? d * post : d, acc[a]);
+                    for (int a = 0; a < decltype(n)::value; ++a) {
+                        int q = pos + rr[a];
+                        if (q >= N) q -= N;
+                        const double d = (double)tile[q * ld + line] - c;
+                        sp_accumulate<PMAX>(Scaled ? d * post : d, acc[a]);
+                    }
                 }
-            }
+            };
+            if (count == 4) run(std::integral_constant<int, 4>{});
+            else if (count == 3) run(std::integral_constant<int, 3>{});
+            else if (count == 2) run(std::integral_constant<int, 2>{});
+            else if (count == 1) run(std::integral_constant<int, 1>{});
         }
     }
+    // the shares' sums meet in shared memory, so that a block adds each sum once
+    double *part = reinterpret_cast<double *>(sp_smem);   // [warp][separation of the group][order]
+    __syncthreads();
 #pragma unroll
     for (int a = 0; a < kSpPerWarp; ++a) {
-        const int m = group * kSpPerWarp + a;
+        if (a >= count) break;
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) {
             const double v = warp_sum(acc[a][p]);
-            if (lane == 0 && m < nr) atomicAdd(Sp + p * nr + m, v);
+            if (lane == 0) part[(warp * kSpPerWarp + a) * PMAX + p] = v;
         }
+    }
+    __syncthreads();
+    const int per_group = kSpPerWarp * PMAX;
+    for (int i = threadIdx.x; i < ngroups * per_group; i += blockDim.x) {
+        const int m = (int)blockIdx.z * ngroups + i / per_group + i % per_group / PMAX * all;
+        if (m >= nr) continue;
+        double v = 0.0;
+        for (int w = 0; w < nwarps; w += ngroups) v += part[w * per_group + i];
+        atomicAdd(Sp + i % PMAX * nr + m, v);
     }
 }
 
@@ -436,7 +462,9 @@ static int sp_sums(Ctx *c, const void *u, size_t stride, int n0, int n1, int n2,
     const int N = c->p.N;
     const bool f64 = c->p.precision == 64;
     const int W = f64 ? sp_lines<double>(N) : sp_lines<float>(N);
-    const size_t shb = (f64 ? sizeof(double) : sizeof(float)) * (size_t)N * (W + 1);
+    // the staged lines, and in their place at the end the warps' sums
+    const size_t shb = std::max((f64 ? sizeof(double) : sizeof(float)) * (size_t)N * (W + 1),
+                                sizeof(double) * (kSpMaxThreads / 32) * kSpPerWarp * 10);
     // The dynamic shared-memory limit is a property of the kernel for the whole process: every
     // context sets the same value, the device's opt-in maximum, so that contexts of different N
     // on concurrent host threads never lower it under another's launch.
@@ -470,16 +498,17 @@ static int sp_sums(Ctx *c, const void *u, size_t stride, int n0, int n1, int n2,
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
     const int64_t tiles = (int64_t)n0 * n1 * n2 / N / W + 1;
-    const int all = (nu + kSpPerWarp - 1) / kSpPerWarp, ngroups = std::min(kSpGroups, all);
-    const unsigned threads = 32u * (unsigned)(ngroups <= 6 ? 2 * ngroups : ngroups);
-    const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)sms * 2)), (unsigned)axes,
-                    (unsigned)((all + kSpGroups - 1) / kSpGroups));
+    const int all = (nu + kSpPerWarp - 1) / kSpPerWarp, nz = (all + kSpGroups - 1) / kSpGroups;
+    const int ngroups = (all + nz - 1) / nz;
+    const int shares = std::min(kSpMaxThreads / 32 / ngroups, std::max(1, N * W / 32 / kSpPositions));
+    const unsigned threads = 32u * (unsigned)(ngroups * shares);
+    const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)sms * 2)), (unsigned)axes, (unsigned)nz);
     const int km = kt_begin(c, KT_STATS);
 #define FWT_SP(REAL, ...)                                                                                          \
 do {                                                                                                           \
     auto k = sp_kernel<REAL, __VA_ARGS__>;                                                                     \
     FWT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));                    \
-    k<<<grid, threads, shb, c->stream>>>((const REAL *)u, stride, N, n0, n1, n2, axis0, (REAL)sc, s, d_r, nu, d_sp); \
+    k<<<grid, threads, shb, c->stream>>>((const REAL *)u, stride, N, n0, n1, n2, axis0, (REAL)sc, s, d_r, nu, ngroups, d_sp); \
 } while (0)
     if (f64) {
         if (!staged) FWT_SP(double, 10, true); else if (P == 4) FWT_SP(double, 4);
