@@ -86,11 +86,13 @@ __global__ void __launch_bounds__(256) pdf_kernel(const Real *__restrict__ a, si
     float *s_hi = (float *)smem;
     float *s_lo = s_hi + nbins;
     uint32_t *s_cnt = (uint32_t *)(s_lo + nbins);
-    for (int i = threadIdx.x; i < nbins; i += blockDim.x) {
+#pragma unroll 8
+    for (int i = threadIdx.x; i < nbins; i += 256) {
         s_hi[i] = hi[i];
         s_lo[i] = lo[i];
     }
-    for (int i = threadIdx.x; i < nbins * copies; i += blockDim.x) s_cnt[i] = 0;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < nbins * copies; i += 256) s_cnt[i] = 0;
     __syncthreads();
     const int mine = (int)threadIdx.x & (copies - 1);
     const float last = s_hi[nbins - 1];
@@ -109,6 +111,10 @@ __global__ void __launch_bounds__(256) pdf_kernel(const Real *__restrict__ a, si
     const size_t nv = n / kV, step = (size_t)gridDim.x * blockDim.x;   // n is a multiple of 8 (N is even)
     const Vec *av = reinterpret_cast<const Vec *>(a);
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (step >= n) {   // a small grid: one value a thread, over as many blocks as that gives
+        if (i < n) count(a[i]);
+        i = nv;
+    }
     for (; i + step < nv; i += 2 * step) {
         const Vec p = av[i], q = av[i + step];
 #pragma unroll
@@ -122,6 +128,12 @@ __global__ void __launch_bounds__(256) pdf_kernel(const Real *__restrict__ a, si
         for (int j = 0; j < kV; ++j) count(p.v[j]);
     }
     __syncthreads();
+    if (copies == 1) {
+#pragma unroll 4
+        for (int i2 = threadIdx.x; i2 < nbins; i2 += 256)
+            if (s_cnt[i2]) atomicAdd(counts + i2, (unsigned long long)s_cnt[i2]);
+        return;
+    }
     for (int i2 = threadIdx.x; i2 < nbins; i2 += blockDim.x) {
         unsigned long long t = 0;
         for (int k = 0; k < copies; ++k) t += s_cnt[i2 * copies + ((k + i2) & (copies - 1))];
@@ -407,9 +419,17 @@ int stats_pdf(Ctx *c, int which, int comp, int nbins, float *val, float *pdf, ui
     FWT_CUDA(cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long) * nbins, c->stream));
     const size_t n3 = field_elems(c);
     const void *f = is_u ? c->b_u.p : c->b_w.p;
-    // copies of the counts: as many as fit 40 KB beside the edges, up to one per lane
+    // the components lie one after the other: one launch takes one of them or all three
+    const size_t o = comp < 0 ? 0 : (size_t)comp * n3, nv = comp < 0 ? 3 * n3 : n3;
+    unsigned grid = grid_for(c, nv, 4);   // a value a thread, where the chip holds as many
+    if ((size_t)grid * 256 < nv) grid = grid_for(c, nv / (c->p.precision == 64 ? 2 : 4), 4);
+    // copies of the counts: as many as fit 40 KB beside the edges, up to one per lane, and no more counts
+    // than a block has values (one component of 32^3, 200 bins, the whole call: 48 us with 16 copies and four
+    // values a thread, 42 so)
     int copies = 1;
-    while (copies < 32 && sizeof(float) * nbins * (2 + 2 * (size_t)copies) <= 40960) copies *= 2;
+    while (copies < 32 && sizeof(float) * nbins * (2 + 2 * (size_t)copies) <= 40960 &&
+           (size_t)nbins * copies * 2 <= nv / grid)
+        copies *= 2;
     const size_t shb = sizeof(float) * 2 * nbins + sizeof(uint32_t) * nbins * (size_t)copies;
     // 8192 bins take 96 KB of shared memory, above the default 48 KB: the limit is raised to
     // the device's opt-in maximum, the same value for every context (the attribute belongs to
@@ -422,14 +442,12 @@ int stats_pdf(Ctx *c, int which, int comp, int nbins, float *val, float *pdf, ui
     else
         FWT_CUDA(cudaFuncSetAttribute(pdf_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     const int km = kt_begin(c, KT_STATS);
-    // the components lie one after the other: one launch takes one of them or all three
-    const size_t o = comp < 0 ? 0 : (size_t)comp * n3, nv = comp < 0 ? 3 * n3 : n3;
     const float ibsz = bsz > 0.0f ? 1.0f / bsz : 0.0f;
     if (c->p.precision == 64)
-        pdf_kernel<double><<<grid_for(c, nv / 2, 4), 256, shb, c->stream>>>((const double *)f + o, nv, s, vmin, ibsz, d_lo,
+        pdf_kernel<double><<<grid, 256, shb, c->stream>>>((const double *)f + o, nv, s, vmin, ibsz, d_lo,
                                                                             d_hi, nbins, copies, d_cnt);
     else
-        pdf_kernel<float><<<grid_for(c, nv / 4, 4), 256, shb, c->stream>>>((const float *)f + o, nv, s, vmin, ibsz, d_lo,
+        pdf_kernel<float><<<grid, 256, shb, c->stream>>>((const float *)f + o, nv, s, vmin, ibsz, d_lo,
                                                                            d_hi, nbins, copies, d_cnt);
     c->launches += 1;
     kt_end(c, km);
