@@ -103,6 +103,10 @@ __device__ __forceinline__ float gelu_d(float x)
 }
 
 constexpr size_t kIoHead = 16;   // bytes of the exchange buffer before x
+// Up to this many bytes the forward pass's outputs come with the flag and the inputs before them, in one
+// copy through the mirror; beyond, in a copy of their own to the caller's place (64 inputs, 256 outputs, us
+// a call, once / apart: 128 rows 90 / 103, 1000 rows 319 / 303, 4096 rows 1110 / 850).
+constexpr size_t kIoOnce = 1 << 19;
 
 // X (B x n_in, FP32) -> X0 (Bp x 64 BF16, zero padded) and its transpose
 __global__ void mlp_pack_input(const float *__restrict__ X, int B, int Bp, int n_in, __nv_bfloat16 *__restrict__ X0,
@@ -824,6 +828,10 @@ int fwt_mlp_forward(fwt_mlp *m, const float *x, int batch, float *y)
     FWT_TRY(mlp_upload(m, x, nullptr, nullptr, batch));
     FWT_TRY(mlp_forward(m, batch, false));
     const size_t nx = m->t_at(batch), ny = (size_t)batch * m->n_out;
+    if (sizeof(float) * (nx + ny) > kIoOnce) {
+        FWT_CUDA(cudaMemcpyAsync(y, m->t(batch), sizeof(float) * ny, cudaMemcpyDeviceToHost, m->st));
+        return mlp_download(m, 0);
+    }
     FWT_TRY(mlp_download(m, nx + ny));
     std::memcpy(y, m->hio + kIoHead + sizeof(float) * nx, sizeof(float) * ny);
     return 0;

@@ -31,3 +31,16 @@ def test_outputs_after_any_input_size(fwt, n_in, n_out, B):
     assert rel_l2(gp, gpo) <= 1e-2
     assert rel_l2(gx, gxo) <= 1e-2
     net.close()
+
+
+@pytest.mark.parametrize("B", [409, 410, 4096])
+def test_outputs_on_both_sides_of_the_single_copy(fwt, B):
+    """Outputs and inputs of up to 2^19 bytes come back in one copy, larger ones apart."""
+    from fastweavturb_b200.surrogate import MLP
+    from oracle import mlp_oracle as MO
+
+    net = MLP(n_in=64, width=64, depth=1, n_out=256, batch_max=4096, seed=6)
+    X = np.random.default_rng(B).uniform(-1, 1, (B, 64)).astype(np.float32)
+    Yo, _, _ = MO.forward(net.params().astype(np.float64), net.widths, X)
+    assert rel_l2(net.forward(X), Yo) <= 1e-3
+    net.close()
