@@ -154,7 +154,7 @@ __device__ __forceinline__ float turning_integrand(const float (&d1)[3][5], cons
 //   2. section_fine_kernel  one thread per listed section: 256 intervals
 //   3. section_kernel       one warp per listed section: the reference's own sum in FP32
 //   4. section_fp64_kernel  one warp per listed section: the reference's sum in FP64
-// Bound by FP32 issue: step 3 takes 1500 warp instructions a section, step 1 about 110.  With every
+// Bound by FP32 issue: step 3 takes 1500 warp instructions a section, step 1 about 145.  With every
 // section in step 3 (and 4) the 38 M sections of a six-level field (H = 0.7) took 68 ms; the four
 // together take 10.0 ms (5.8, 2.6, 1.0, 0.6).
 //

@@ -94,7 +94,7 @@ __global__ void piece_map_kernel(const LineParam *__restrict__ lp, const int *__
 // thread, most of 4 bytes, became 47 of 16.  4.2 M pieces: 2.57 -> 2.16 ms.  (Eight lanes to a piece,
 // the samples from their neighbours and the record out of shared memory: 2.8 ms, 2.5 times the
 // instructions.)
-constexpr int kBuildThreads = 64;   // piece_build_kernel's block: 32 KB of shared memory, six per SM
+constexpr int kBuildThreads = 64;   // piece_build_kernel's block: 36 KB of shared memory, six per SM
 __global__ void __launch_bounds__(kBuildThreads, 6) piece_build_kernel(
     const LineParam *__restrict__ lp, const int *__restrict__ slot_line, const int *__restrict__ map, int64_t npieces,
     const double *__restrict__ X, const double *__restrict__ Y, const double *__restrict__ Z,
