@@ -87,18 +87,20 @@ __global__ void __launch_bounds__(kDepThreads, Policy::kCtas) deposit_block_kern
     const int nrec = (int)(c1 - c0);
     const int nchunks = (nrec + Policy::kChunk - 1) / Policy::kChunk;
 
-    // warp 0: expect the chunk's bytes, then one bulk copy per record
+    // warp 0: the chunk's record ids, then one bulk copy per record.  The ids are plain stores, and what
+    // the other warps wait for is the mbarrier: they are written before lane 0 arrives on it (a release,
+    // which the wait's acquire meets; the copies' bytes alone would not publish them).  A barrier after the
+    // sums' set-up does it too, but spills registers: 512^3, radius 122 to 15: 307 ms, 296 so.
     auto issue = [&](int ch) {
         const int b = ch & 1;
         const int64_t base = c0 + (int64_t)ch * Policy::kChunk;
         const int nc = min(Policy::kChunk, nrec - ch * Policy::kChunk);
+        for (int t = lane; t < nc; t += 32) S.id[b][t] = __ldg(list + base + t);
+        __syncwarp();
         if (lane == 0) mbar_expect(&S.bar[b], (uint32_t)(nc * sizeof(typename Policy::Rec)));
         __syncwarp();
-        for (int t = lane; t < nc; t += 32) {
-            const uint32_t v = __ldg(list + base + t);
-            S.id[b][t] = v;
-            bulk_g2s(&S.rec[b][t], rec + (v & ((1u << 26) - 1u)), (uint32_t)sizeof(typename Policy::Rec), &S.bar[b]);
-        }
+        for (int t = lane; t < nc; t += 32)
+            bulk_g2s(&S.rec[b][t], rec + (S.id[b][t] & ((1u << 26) - 1u)), (uint32_t)sizeof(typename Policy::Rec), &S.bar[b]);
     };
     if (tid == 0) {
         mbar_init(&S.bar[0]);
@@ -136,9 +138,6 @@ __global__ void __launch_bounds__(kDepThreads, Policy::kCtas) deposit_block_kern
         acc[1][pa] = a1;
         acc[2][pa] = a2;
     }
-    // the first chunk's record ids, written by warp 0 with plain stores, are read by every warp (the
-    // barriers of the chunk loop order the later ones; the mbarrier orders the bulk copies alone)
-    __syncthreads();
 
     // an emit-only pass lists the deferred pairs again and discards its sums
     const float fscale = D.emit_only ? 0.0f : (float)scale;
