@@ -154,9 +154,9 @@ __device__ __forceinline__ float turning_integrand(const float (&d1)[3][5], cons
 //   2. section_fine_kernel  one thread per listed section: 256 intervals
 //   3. section_kernel       one warp per listed section: the reference's own sum in FP32
 //   4. section_fp64_kernel  one warp per listed section: the reference's sum in FP64
-// Bound by FP32 issue: step 3 takes 1500 warp instructions a section, step 1 about 145.  With every
+// Bound by FP32 issue: step 3 takes 1500 warp instructions a section, step 1 a tenth.  With every
 // section in step 3 (and 4) the 38 M sections of a six-level field (H = 0.7) took 68 ms; the four
-// together take 10.0 ms (5.8, 2.6, 1.0, 0.6).
+// together take 9.4 ms (5.3, 2.5, 1.0, 0.6).
 //
 // The bound.  Simpson's rule over 2h is off by the integral of f'' times a kernel that is at most h^2/6,
 // and a second difference is h f'' averaged over a hat of that width: h / 6 sum |second differences|
@@ -183,8 +183,8 @@ constexpr int kQuadMinPre = 512;
 // Quadratures before step 3: 0 none, 1 the 64 intervals, 2 both.  A thread walks its intervals in a
 // chain, 5 us for 64 of them and 20 for 256 however few sections there are, while step 3 has a warp for
 // each: few sections go to it at once.  All steps, us, with 0 / 1 / 2 (fractional bridges, H = 0.3):
-// 1,028 slots 30 / 35 / 58, 4,112 44 / 45 / 66, 16,448 64 / 50 / 69, 65,792 161 / 80 / 84, 131,584
-// 293 / 125 / 110.
+// 1,028 slots 30 / 34 / 54, 4,112 44 / 44 / 62, 16,448 64 / 49 / 64, 65,792 163 / 79 / 80, 131,584
+// 292 / 123 / 104.
 inline int section_coarse(int ntf_pre, int64_t slots)
 {
     if (ntf_pre < kQuadMinPre || slots <= (1 << 12)) return 0;
@@ -201,36 +201,38 @@ template <int Intervals>
 __device__ __forceinline__ SectionSum section_quadrature(const float (&d1)[3][5], const float (&d2)[3][4], float zr,
                                                          int ntf_pre)
 {
+    static_assert(Intervals % 32 == 0, "section_quadrature");
     const float h = 1.0f / Intervals, dz = zr * h;
     float q0, q1, q2;
     float f0 = turning_integrand(d1, d2, 0.0f, q0), f1 = turning_integrand(d1, d2, dz, q1);
     const float fa = f0, qa = q0;
-    double sum = 0.0;                         // 4 x odd + 2 x even samples
-    float odd = f1, even = 0.0f, dd = 0.0f;   // of up to 32 of them; sum of |second differences|
-    float qx = 0.0f;                          // the first end's second difference
+    double sum = 0.0;            // 4 x odd + 2 x even samples
+    float dd = 0.0f, e = 0.0f;   // sum of |second differences|; |c'|^2's second difference
     bool rough = false;
-#pragma unroll 2
-    for (int i = 2; i <= Intervals; ++i) {
-        const float f2 = turning_integrand(d1, d2, dz * (float)i, q2);
+    // sample n into its sum, and the second differences about it
+    auto sample = [&](int n, float &side) {
+        const float f2 = turning_integrand(d1, d2, dz * (float)(n + 1), q2);
         dd += fabsf((f0 - f1) + (f2 - f1));
-        const float e = (q0 - q1) + (q2 - q1);
+        e = (q0 - q1) + (q2 - q1);
         rough = rough || !(e <= 0.1f * q1);
-        if (i == 2) qx = e;
-        if (i == Intervals) rough = rough || !(e <= 0.1f * q2);
-        if (i < Intervals) {
-            if (i & 1) odd += f2;
-            else even += f2;
-            if (i % 32 == 31) {
-                sum += 4.0 * (double)odd + 2.0 * (double)even;
-                odd = even = 0.0f;
-            }
-        }
+        side += f1;
         f0 = f1;
         f1 = f2;
         q0 = q1;
         q1 = q2;
+    };
+#pragma unroll 1
+    for (int b = 0; b < Intervals; b += 32) {
+        float odd = 0.0f, even = 0.0f;
+#pragma unroll 2
+        for (int n = b + 1; n < b + 33; n += 2) {
+            sample(n, odd);
+            if (n == 1) rough = rough || !(e <= 0.1f * qa);
+            if (n + 1 < Intervals) sample(n + 1, even);
+        }
+        sum += 4.0 * (double)odd + 2.0 * (double)even;
     }
-    rough = rough || !(qx <= 0.1f * qa);
+    rough = rough || !(e <= 0.1f * q1);
     SectionSum s;
     // n_pre times Simpson's integral over the unit interval, plus half the end values
     const double ends = (double)fa + (double)f1;
