@@ -145,14 +145,14 @@ __global__ void __launch_bounds__(256) pdf_kernel(const Real *__restrict__ a, si
 // as [pos][line] (padded), in the field's own precision; groups at the end of an axis may hold
 // fewer lines, so any N works.  axis 0: u_x along x; 1: u_y along y; 2: u_z along z.
 //
-// Bound by FP64 arithmetic: the sums of du^p, p = 1..PMAX, over every point and separation.  A
-// warp takes MPW separations and a share of the positions, so a point is read and widened once
-// for MPW increments; the sums use the even powers and fused multiply-adds (8 FP64 operations
-// for p <= 6, 14 for 10, where a running power took 21), the scale s = 1/u' enters as the power of
-// two just above it, exactly, when the lines are staged, and as the remainder in [0.5, 1) at the end,
-// only as many orders as asked for are summed, and separations equal modulo N once (the host's list).  512^3, three
-// components, orders 1-6: 14.5 ms with the running power to order 10, 6.8 now; at the FP64 rate
-// the 17 separations take 3.8.
+// Bound by FP64 arithmetic (the sums of du^p, p = 1..PMAX, over every point and separation) and by the
+// staging of the lines, which nothing overlaps.  A warp takes up to four separations and a share of the
+// positions, so a point is read and widened once for four increments; the sums use the even powers and
+// fused multiply-adds (8 FP64 operations for p <= 6, 14 for 10, where a running power took 21), the scale
+// s = 1/u' enters as the power of two just above it, exactly, when the lines are staged, and as the
+// remainder in [0.5, 1) at the end, only as many orders as asked for are summed, and separations equal
+// modulo N once (the host's list).  512^3, three components, orders 1-6: 14.5 ms with the running power to
+// order 10, 6.8 now; at the FP64 rate the 17 separations take 3.8.
 template <typename Real>
 __host__ __device__ constexpr int sp_lines(int N)
 {
@@ -161,11 +161,11 @@ __host__ __device__ constexpr int sp_lines(int N)
 constexpr int kSpPerWarp = 4;   // separations of a warp at the most
 static_assert(kSpPerWarp == 4, "sp_kernel's loops");
 // Groups of separations in a block, and its threads.  The groups are spread evenly over as few blocks as
-// hold them, a group takes three or four separations (fewer only where there are fewer), and few groups
-// share the positions among several warps each.  With up to eight groups in the first block, four
-// separations in each whether asked for or not, and two warps a group, few separations took longer than
-// with one warp for every eighth: 512^3, ms (and with running powers): one separation, orders
-// 1-6: 7.9 -> 1.7 (5.3), 33, orders 1-10: 34.3 -> 21.2 (28.7), 17, orders 1-6: 7.8 -> 6.8 (13.6).
+// hold them, and so are the separations over the groups; few groups share the positions among several
+// warps each.  When a block took eight groups of four whether asked for or not, two warps to a group at
+// the most, few separations took longer than with one warp each: 512^3, ms, so / now (one warp each): one
+// separation, orders 1-6: 7.9 / 1.7 (5.3); 33, orders 1-10: 34.3 / 21.2 (28.7); 17, orders 1-6: 7.8 / 6.8
+// (13.6).
 constexpr int kSpGroups = 8, kSpMaxThreads = 384;
 constexpr int kSpPositions = 16;   // positions a lane at the least, where positions are shared
 
@@ -198,9 +198,9 @@ __device__ __forceinline__ void sp_accumulate(double d, double (&acc)[PMAX])
 // The field is a box n0 x n1 x n2 (x fastest) whose extent along the axis is the line length N:
 // the whole grid, or a z-slab (axes 0, 1) or y-pencil (axis 2) of a grid split over GPUs.  The
 // axis is axis0 + blockIdx.y, its component stride elements further on per step.  blockDim is
-// 32 x (groups of separations) x (shares of the positions); blockIdx.z takes the next groups.  Scaled: each increment is multiplied by `post` in FP64, for a
-// scale that says nothing about the field's size (a caller's own, or one beyond the staged type's
-// exponents), where sc is 1.
+// 32 x (groups of separations) x (shares of the positions); blockIdx.z takes the next groups.
+// Scaled: each increment is multiplied by `post` in FP64, for a scale that says nothing about the
+// field's size (a caller's own, or one beyond the staged type's exponents), where sc is 1.
 template <typename Real, int PMAX, bool Scaled = false>
 __global__ void __launch_bounds__(kSpMaxThreads, PMAX > 6 ? 1 : 2) sp_kernel(const Real *__restrict__ u0, size_t stride, int N, int n0, int n1, int n2,
                                                  int axis0, Real sc, double post, const int *__restrict__ rs,
