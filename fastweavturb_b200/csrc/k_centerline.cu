@@ -242,13 +242,18 @@ __device__ __forceinline__ SectionSum section_quadrature(const float (&d1)[3][5]
     return s;
 }
 
+// The scaled angle of a section that can be sub-divided: more sub-segments than a batch may hold, or an
+// angle that is not a number (consecutive nodes that coincide, a coordinate that is not finite), would
+// take the records out of bounds, and is refused after the last step (SectionLists::bad).
+constexpr double kMaxSubSegs = 67108864.0;   // 2^26
+
 // Decide a slot from its sum, or leave it to the next list: 0 decided, 1 the quadrature's bound
 // straddles a step, 2 only the FP32 rounding (1e-4) does.
 __device__ __forceinline__ int section_decide(const SectionSum &q, double dtfp, double L, int ntf_times, int &ntf)
 {
     const double k = dtfp * L * ntf_times / dev_pi2();
     const double x = q.tsum * k, rounding = 1e-4 * (x + 1.0), e = (double)q.err * k;
-    if (!q.resolved || !(x == x) || !(e == e)) return 1;
+    if (!q.resolved || !(x < kMaxSubSegs) || !(e == e)) return 1;
     const double m = e + rounding;
     if (floor(x + m) == floor(x - m)) {
         ntf = (int)ceil(x) + 1;
@@ -260,6 +265,7 @@ __device__ __forceinline__ int section_decide(const SectionSum &q, double dtfp, 
 // The lists of undecided slots: three of them, each its counter and its slots.
 struct SectionLists {
     unsigned *count;        // [0] fine, [1] full sum, [2] FP64
+    int64_t *bad;           // sections without a count
     unsigned *fine, *full, *fp64;
 };
 
@@ -420,7 +426,7 @@ __global__ void __launch_bounds__(256) section_kernel(const LineParam *__restric
             const double dtfp = (zr_ - zl) / (1.0 * ntf_pre);
             const double xr = ntf_times * (sum * dtfp * Len[l]) / dev_pi2();
             const double fr = xr - floor(xr);
-            const bool near_step = fmin(fr, 1.0 - fr) < 1e-4 * (xr + 1.0) || !(xr == xr);
+            const bool near_step = fmin(fr, 1.0 - fr) < 1e-4 * (xr + 1.0) || !(xr < kMaxSubSegs);
             if (near_step) {
                 lists.fp64[atomicAdd(lists.count + 2, 1u)] = (unsigned)s;
             } else {
@@ -474,7 +480,10 @@ __global__ void section_fp64_kernel(const LineParam *__restrict__ lp, const int 
         }
         th = warp_sum(th);
         if (lane == 0) {
-            const int ntf = (int)ceil(ntf_times * th / dev_pi2()) + 1;
+            const double x = ntf_times * th / dev_pi2();
+            const bool counted = x < kMaxSubSegs;
+            if (!counted) atomicAdd((unsigned long long *)lists.bad, 1ull);
+            const int ntf = counted ? (int)ceil(x) + 1 : 1;
             ntf_out[warp] = ntf;
             dtf_out[warp] = (zr_ - zl) / (1.0 * ntf);
         }
@@ -1005,6 +1014,8 @@ int centerline_setup(Ctx *c, int la, int lb, CenterlineBatch &B, BatchRecords mo
     lists.fine = lists.count + 4;
     lists.full = lists.fine + slots;
     lists.fp64 = lists.full + slots;
+    lists.bad = d_misc + 2 * nl + 2;
+    FWT_CUDA(cudaMemsetAsync(lists.bad, 0, sizeof(int64_t), c->stream));
     FWT_CUDA(cudaMemsetAsync(lists.count, 0, 4 * sizeof(unsigned), c->stream));
     FWT_TRY(buf_reserve(c, C.scratch[28], sizeof(float) * (size_t)std::max<int64_t>(slots, 1)));
     float *d_zstep = (float *)C.scratch[28].p;
@@ -1036,11 +1047,16 @@ int centerline_setup(Ctx *c, int la, int lb, CenterlineBatch &B, BatchRecords mo
     FWT_TRY(scan_exclusive_i64(c, B.qoff, slots, d_misc + 2 * nl + 1, C.scratch[13]));
     kt_end(c, km);
     // per-line Len and ntf statistics + totals to the host
-    std::vector<int64_t> hmisc((size_t)(2 * nl + 2));
+    std::vector<int64_t> hmisc((size_t)(2 * nl + 3));
     std::vector<double> hLen((size_t)nl);
-    FWT_CUDA(cudaMemcpyAsync(hmisc.data(), d_misc, sizeof(int64_t) * (2 * nl + 2), cudaMemcpyDeviceToHost, c->stream));
+    FWT_CUDA(cudaMemcpyAsync(hmisc.data(), d_misc, sizeof(int64_t) * (2 * nl + 3), cudaMemcpyDeviceToHost, c->stream));
     FWT_CUDA(cudaMemcpyAsync(hLen.data(), B.Len, sizeof(double) * nl, cudaMemcpyDeviceToHost, c->stream));
     FWT_CUDA(cudaStreamSynchronize(c->stream));
+    if (hmisc[2 * nl + 2] != 0)
+        return fail(FWT_E_RANGE, "lines " + std::to_string(la + 1) + ".." + std::to_string(lb) + ": " +
+                                     std::to_string(hmisc[2 * nl + 2]) +
+                                     " sections cannot be sub-divided (consecutive nodes that coincide, or a "
+                                     "coordinate that is not finite?)");
     B.nsamples = hmisc[2 * nl];
     B.nsub = hmisc[2 * nl + 1];
     B.line_ntf_sum.assign(hmisc.begin(), hmisc.begin() + 2 * nl);
